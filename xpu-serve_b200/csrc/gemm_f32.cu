@@ -1,0 +1,294 @@
+// out[M, N] = x[M, K] . w[N, K]^T (+ bias[N]) in float32 on CUDA-core FMAs: the float32 path's product where rows start on
+// 16-byte boundaries (gemm_generic.cu keeps the other cases and the element types).
+//
+// Order of the sums: 32 consecutive k into a partial by fused multiply-adds in ascending k, partials added in ascending k, for
+// every output and in every kernel here. It is the order of gemm_generic.cu, so a row's result is the same bit for bit whatever
+// the other rows of the call are, and whichever kernel takes them.
+//
+// Two kernels:
+//   few rows (up to 64, 4, 8 or 16 at a time): bound by the weights' bytes. A CTA takes 8 weight rows at a time and streams them
+//     past x in stages of 1,024 k (cp.async, two stages, a 16-byte piece of every row a thread), a thread multiplying one 32-k chunk
+//     of one weight row. The chunks' partials meet in shared memory, where one thread an output adds them in order while the next
+//     stage is multiplied. Weight rows' 16-byte pieces are swizzled by row, x's by chunk, so that neither load has bank conflicts.
+//     (With 128 threads, stages of 512 k and one or two weight rows a thread the SM had one warp a scheduler: 2.0 TB/s.)
+//   more rows: bound by the FMA units. 64 x 128 outputs a CTA of 128 threads, 8 x 8 a thread, both operands in stages of 32 k as
+//     they lie in memory (rows of k, 36 floats apart: the eight rows of a 16-byte load's phase fall into different banks), so
+//     nothing is transposed; a stage is exactly one partial.
+//
+// Measured on B200 (products of the 350M shape, weights from memory, us; before: the 64 x 64 tile of gemm_generic.cu, whose time
+// does not depend on the rows):
+//     N 13312 K 1024    4 rows 210 -> 13.5 (4.0 TB/s)   16 rows 212 -> 32   64 rows 221 -> 107   1,294 rows 1,569 -> 852 (41 TFLOP/s)
+//     N  1024 K 6656    4 rows 1,218 -> 14.7            16 rows 1,232 -> 20   64 rows 1,264 -> 72   1,294 rows 1,144 -> 735
+//     N 65536 K 1024    4 rows 462 -> 52 (5.2 TB/s)     16 rows 464 -> 140
+#include "common.cuh"
+
+namespace {
+
+constexpr int kChunk = 32;            // k of one partial sum
+constexpr int kStages = 3;            // of the tile kernel
+constexpr int kFewThreads = 256, kFewRows = 8;      // few rows: threads and weight rows a CTA
+constexpr int kStageK = 4 * kFewThreads;            // few rows: k of a stage, a 16-byte piece of every row a thread
+constexpr int kFewRowsMost = 64;
+
+__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// 16 bytes, of which the first `bytes` (0 to 16) are read and the rest are zeros.
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Up to MR rows of x.
+template <int MR>
+__global__ void __launch_bounds__(kFewThreads, MR <= 4 ? 2 : 1)
+gemm_f32_few_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+                         float* __restrict__ out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo) {
+    constexpr int kChunks = kStageK / kChunk;                     // 32
+    constexpr int kStageFloats = (kFewRows + MR) * kStageK;
+    constexpr int kOuts = kFewRows * MR;                          // 32, 64 or 128: at most one a thread
+    extern __shared__ __align__(16) float sm[];
+    float* parts = sm + 2 * kStageFloats;                         // [2][kChunks][MR][kFewRows]
+    const int m0 = blockIdx.y * MR;
+    const int r = threadIdx.x & 7, c = threadIdx.x >> 3;          // a thread multiplies chunk c of weight row r
+    // and copies the 16-byte piece r of chunk c of every row: its place in a row of the stage, for weight rows turned by the row
+    const int piece = threadIdx.x * 4;
+    pdl_launch_dependents();
+    const int stages = (K + kStageK - 1) / kStageK;
+    const int tiles = (N + kFewRows - 1) / kFewRows;
+    // the CTA's tiles are walked as one run of stages: the next tile's weights are on their way while this one's are multiplied
+    const int total = ((tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * stages;
+    auto load_w = [&](float* stage, int n0, int k0) {
+        const int bytes = min(16, max(0, (K - k0 - piece) * 4));
+        const float* from = w + (int64_t)n0 * ldw + k0 + piece;
+        const uint32_t to = smem_at(stage + c * kChunk);
+#pragma unroll
+        for (int q = 0; q < kFewRows; ++q) {
+            const int there = n0 + q < N ? bytes : 0;
+            copy16(to + (uint32_t)(q * kStageK + ((r ^ q) << 2)) * 4u, there > 0 ? from + (int64_t)q * ldw : w, there);
+        }
+    };
+    auto load_x = [&](float* stage, int k0) {
+        const int bytes = min(16, max(0, (K - k0 - piece) * 4));
+        const float* from = x + (int64_t)m0 * ldx + k0 + piece;
+        const uint32_t to = smem_at(stage + kFewRows * kStageK + c * kChunk + ((r ^ (c & 7)) << 2));
+#pragma unroll
+        for (int q = 0; q < MR; ++q) {
+            const int there = m0 + q < M ? bytes : 0;
+            copy16(to + (uint32_t)(q * kStageK) * 4u, there > 0 ? from + (int64_t)q * ldx : x, there);
+        }
+    };
+    int load_n = blockIdx.x * kFewRows, load_s = 0;               // the stage to be asked for next
+    auto next_load = [&] {
+        if (++load_s == stages) {
+            load_s = 0;
+            load_n += gridDim.x * kFewRows;
+        }
+    };
+    if (total > 0) load_w(sm, load_n, 0);
+    pdl_wait();                                                   // x is written by the kernel before this one
+    if (total > 0) load_x(sm, 0);
+    copies_commit();
+    next_load();
+    float acc = 0.0f;
+    int n0 = blockIdx.x * kFewRows, s_at = 0;                     // the stage whose partials are added next
+    // adds a stage's partials; behind a tile's last stage, stores its outputs
+    auto add_parts = [&](const float* from) {
+        const int o = threadIdx.x;
+        if (o < kOuts) {
+#pragma unroll
+            for (int j = 0; j < kChunks; ++j) acc += from[j * kOuts + o];
+            if (s_at == stages - 1) {
+                const int m = m0 + o / kFewRows, n = n0 + o % kFewRows;
+                if (m < M && n < N) out[(int64_t)m * ldo + n] = bias != nullptr ? acc + bias[n] : acc;
+                acc = 0.0f;
+            }
+        }
+        if (++s_at == stages) {
+            s_at = 0;
+            n0 += gridDim.x * kFewRows;
+        }
+    };
+    for (int g = 0; g < total; ++g) {
+        copies_wait<0>();
+        __syncthreads();                      // stage g is here, stage g - 1 has been read, its partials are written
+        if (g + 1 < total) {
+            float* to = sm + ((g + 1) & 1) * kStageFloats;
+            load_w(to, load_n, load_s * kStageK);
+            load_x(to, load_s * kStageK);
+            next_load();
+        }
+        copies_commit();
+        const float* ws = sm + (g & 1) * kStageFloats + r * kStageK + c * kChunk;
+        const float* xs = sm + (g & 1) * kStageFloats + kFewRows * kStageK + c * kChunk;
+        float part[MR];
+#pragma unroll
+        for (int m = 0; m < MR; ++m) part[m] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kChunk / 4; ++i) {
+            const float4 b = *reinterpret_cast<const float4*>(ws + ((i ^ r) << 2));
+            float4 a[MR];
+#pragma unroll
+            for (int m = 0; m < MR; ++m) a[m] = *reinterpret_cast<const float4*>(xs + m * kStageK + ((i ^ (c & 7)) << 2));
+#pragma unroll
+            for (int m = 0; m < MR; ++m) part[m] = fmaf(a[m].x, b.x, part[m]);
+#pragma unroll
+            for (int m = 0; m < MR; ++m) part[m] = fmaf(a[m].y, b.y, part[m]);
+#pragma unroll
+            for (int m = 0; m < MR; ++m) part[m] = fmaf(a[m].z, b.z, part[m]);
+#pragma unroll
+            for (int m = 0; m < MR; ++m) part[m] = fmaf(a[m].w, b.w, part[m]);
+        }
+        if (g > 0) add_parts(parts + ((g - 1) & 1) * kChunks * kOuts);
+        float* to = parts + ((g & 1) * kChunks + c) * kOuts + r;
+#pragma unroll
+        for (int m = 0; m < MR; ++m) to[m * kFewRows] = part[m];
+    }
+    __syncthreads();
+    if (total > 0) add_parts(parts + ((total - 1) & 1) * kChunks * kOuts);
+}
+
+constexpr int BM = 64, kRow = kChunk + 4;
+
+template <int BN>
+__global__ void __launch_bounds__(BN, 256 / BN)
+gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+                     float* __restrict__ out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr int kTileFloats = (BM + BN) * kRow, TX = BN / 8;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+    const int stages = (K + kChunk - 1) / kChunk;
+    // a thread copies the piece tid & 7 of the rows tid / 8, + TX, + 2 TX, ... of each operand
+    const int piece = threadIdx.x & 7, row = threadIdx.x >> 3;
+    auto load = [&](int s, bool weights, bool inputs) {
+        float* to = sm + (s % kStages) * kTileFloats;
+        const int k = s * kChunk + piece * 4;
+        const int left = min(16, max(0, (K - k) * 4));
+        if (inputs) {
+#pragma unroll
+            for (int q = 0; q < BM / TX; ++q) {
+                const int m = m0 + row + TX * q;
+                const int n_bytes = m < M ? left : 0;
+                copy16(smem_at(to + (row + TX * q) * kRow + piece * 4), n_bytes > 0 ? x + (int64_t)m * ldx + k : x, n_bytes);
+            }
+        }
+        if (weights) {
+#pragma unroll
+            for (int q = 0; q < BN / TX; ++q) {
+                const int n = n0 + row + TX * q;
+                const int n_bytes = n < N ? left : 0;
+                copy16(smem_at(to + (BM + row + TX * q) * kRow + piece * 4), n_bytes > 0 ? w + (int64_t)n * ldw + k : w, n_bytes);
+            }
+        }
+    };
+    pdl_launch_dependents();
+#pragma unroll
+    for (int s = 0; s < kStages - 1; ++s)
+        if (s < stages) load(s, true, false);
+    pdl_wait();
+#pragma unroll
+    for (int s = 0; s < kStages - 1; ++s) {
+        if (s < stages) load(s, false, true);
+        copies_commit();
+    }
+    float acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+    for (int s = 0; s < stages; ++s) {
+        copies_wait<kStages - 2>();
+        __syncthreads();
+        if (s + kStages - 1 < stages) load(s + kStages - 1, true, true);
+        copies_commit();
+        const float* xs = sm + (s % kStages) * kTileFloats + ty * kRow;
+        const float* ws = sm + (s % kStages) * kTileFloats + (BM + tx) * kRow;
+        float part[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) part[i][j] = 0.0f;
+#pragma unroll 2
+        for (int k = 0; k < kChunk; k += 4) {
+            float4 a[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(xs + 8 * i * kRow + k);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float4 b = *reinterpret_cast<const float4*>(ws + TX * j * kRow + k);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].x, b.x, part[i][j]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].y, b.y, part[i][j]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].z, b.z, part[i][j]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].w, b.w, part[i][j]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] += part[i][j];
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + ty + 8 * i;
+        if (m >= M) continue;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int n = n0 + tx + TX * j;
+            if (n < N) out[(int64_t)m * ldo + n] = bias != nullptr ? acc[i][j] + bias[n] : acc[i][j];
+        }
+    }
+}
+
+template <int MR>
+cudaError_t launch_few(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int64_t ldx, int64_t ldw,
+                       int64_t ldo, cudaStream_t stream) {
+    const size_t smem = (2 * (size_t)(kFewRows + MR) * kStageK + 2 * (kStageK / kChunk) * kFewRows * MR) * sizeof(float);
+    static const cudaError_t opted =
+        cudaFuncSetAttribute(gemm_f32_few_rows_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (opted != cudaSuccess) return opted;
+    const int tiles = ceil_div_i(N, kFewRows), chunks = ceil_div_i(M, MR);
+    const int fit = 148 * (smem <= 110 * 1024 ? 2 : 1);           // CTAs that are resident at one time
+    return xs_launch(gemm_f32_few_rows_kernel<MR>, dim3(tiles < fit ? tiles : fit, chunks), dim3(kFewThreads), smem, stream, x, w, bias,
+                     out, M, N, K, ldx, ldw, ldo);
+}
+
+template <int BN>
+cudaError_t launch_tile(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int64_t ldx, int64_t ldw,
+                        int64_t ldo, cudaStream_t stream) {
+    const size_t smem = (size_t)kStages * (BM + BN) * kRow * sizeof(float);
+    static const cudaError_t opted = cudaFuncSetAttribute(gemm_f32_tile_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (opted != cudaSuccess) return opted;
+    return xs_launch(gemm_f32_tile_kernel<BN>, dim3(ceil_div_i(N, BN), ceil_div_i(M, BM)), dim3(BN), smem, stream, x, w, bias, out, M, N, K,
+                     ldx, ldw, ldo);
+}
+
+}  // namespace
+
+// Whether the kernels here take a product: rows that start on 16-byte boundaries.
+bool xs_gemm_f32_takes(const void* x, const void* w, int64_t ldx, int64_t ldw) {
+    return (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0 && ldx % 4 == 0 && ldw % 4 == 0;
+}
+
+int xs_gemm_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int64_t ldx, int64_t ldw,
+                int64_t ldo, cudaStream_t stream) {
+    cudaError_t e;
+    // (between 17 and 64 rows: the tiles where they are enough to fill half of the device's SMs)
+    if (M <= 16 || (M <= kFewRowsMost && ceil_div_i(N, 64) < 74)) {
+        e = M <= 4 ? launch_few<4>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream)
+            : M <= 8 ? launch_few<8>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream)
+                     : launch_few<16>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream);
+    } else {
+        XS_REQUIRE(ceil_div_i(M, BM) <= 65535, "gemm: %d rows exceed the grid limit", M);
+        // the wide tile reads less from shared memory a product; the narrow one where it would leave less than three CTAs an SM
+        const int64_t wide = (int64_t)ceil_div_i(M, BM) * ceil_div_i(N, 128);
+        e = wide >= 3 * 148 ? launch_tile<128>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream)
+                            : launch_tile<64>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream);
+    }
+    XS_REQUIRE(e == cudaSuccess, "gemm (float32): launch failed: %s", cudaGetErrorString(e));
+    return 0;
+}

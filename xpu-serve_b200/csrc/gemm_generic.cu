@@ -9,6 +9,11 @@
 // (src/graph/graph.h:12,46).
 #include "common.cuh"
 
+// gemm_f32.cu: float32 operands whose rows start on 16-byte boundaries
+bool xs_gemm_f32_takes(const void* x, const void* w, int64_t ldx, int64_t ldw);
+int xs_gemm_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int64_t ldx, int64_t ldw,
+                int64_t ldo, cudaStream_t stream);
+
 namespace {
 
 constexpr int TM = 64, TN = 64, TK = 32;
@@ -82,6 +87,8 @@ XS_API int xs_gemm_generic(const void* x, const void* w, const float* bias, void
     if (M == 0 || N == 0) return 0;
     XS_REQUIRE(M > 0 && N > 0 && K > 0, "gemm: sizes %d x %d x %d", M, N, K);
     XS_REQUIRE(ldx >= K && ldw >= K && ldo >= N, "gemm: a row stride is shorter than its row");
+    if (in_dtype == XS_F32 && out_dtype == XS_F32 && xs_gemm_f32_takes(x, w, ldx, ldw))
+        return xs_gemm_f32((const float*)x, (const float*)w, bias, (float*)out, M, N, K, ldx, ldw, ldo, stream);
     const dim3 grid(ceil_div_i(N, TN), ceil_div_i(M, TM));
     XS_REQUIRE(grid.y <= 65535, "gemm: %d rows exceed the grid limit", M);
     if (in_dtype == XS_F32 && out_dtype == XS_F32) {
