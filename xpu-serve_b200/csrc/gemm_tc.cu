@@ -35,6 +35,7 @@ namespace {
 constexpr int BM = 128;          // weight rows per tile (MMA M)
 constexpr int BK = 64;           // k per stage: one 128-byte swizzle atom of bfloat16
 constexpr int kThreads = 192;    // producer warp, MMA warp, four epilogue warps
+constexpr int kManyThreads = 320;    // the many-token kernels: eight epilogue warps, two for each quarter of tensor memory's lanes
 
 enum Epilogue : int { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_SWIGLU = 2, EPI_RELU_SQ = 3 };     // 3: store max(v, 0)^2
 
@@ -45,7 +46,7 @@ struct GemmTcParams {
     unsigned int* counters;   // [tiles_m * tiles_n], zero between calls
     int* status;              // set non-zero when a wait gave up
     int T, N, K, ksplit, epilogue, out_f32;
-    int vec;                  // rows of out start on 16-byte boundaries: the many-token epilogue may store vectors
+    int vec;                  // rows of out start on 16-byte boundaries: the many-token epilogue may store vectors (2: on 32-byte ones)
     int64_t ldo;
     // the gated epilogue's activation: limit 0: silu(gate) * up; limit > 0: g = min(gate, limit), u = clamp(up, -limit, limit),
     // g * sigmoid(alpha g) * (u + shift)
@@ -53,15 +54,23 @@ struct GemmTcParams {
     int glu_act;              // 1: the gate passes the tanh form of gelu instead (no limit)
 };
 
+// 1 / v to one unit in the last place, by the hardware's reciprocal (the division's own steps for odd ranges and the last half
+// unit cost the gated epilogue a third of its instructions, for a result that is rounded to bfloat16).
+__device__ __forceinline__ float near_rcp(float v) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 __device__ __forceinline__ float gated_unit(const GemmTcParams& p, float g, float u) {
     // (0.5 (1 + tanh(a)) = 1 / (1 + exp(-2 a)): the tanh form of gelu costs one exponential, as silu does)
     if (p.glu_act == 1) return __fdividef(g * u, 1.0f + __expf(-1.5957691216057308f * g * fmaf(0.044715f * g, g, 1.0f)));
     if (p.glu_limit > 0.0f) {
         g = fminf(g, p.glu_limit);
         u = fminf(fmaxf(u, -p.glu_limit), p.glu_limit);
-        return g / (1.0f + __expf(-p.glu_alpha * g)) * (u + p.glu_shift);
+        return g * near_rcp(1.0f + __expf(-p.glu_alpha * g)) * (u + p.glu_shift);
     }
-    return g / (1.0f + __expf(-g)) * u;
+    return g * near_rcp(1.0f + __expf(-g)) * u;
 }
 
 // Instruction descriptor of this file's single-CTA products: M = 128, N = n.
@@ -173,6 +182,67 @@ __device__ __forceinline__ void emit16(const GemmTcParams& p, const uint32_t* r,
 #pragma unroll
         for (int j = 0; j < 16; ++j)
             if (f0 + j < p.N) o[j] = __float2bfloat16_rn(v[j]);
+    }
+}
+
+// Thirty-two of them (f0 a multiple of 32), in whole 32-byte sectors where the rows allow it.
+__device__ __forceinline__ void emit32(const GemmTcParams& p, const uint32_t* r, int token, int f0) {
+    if (p.vec < 2 || p.bias != nullptr || f0 + 32 > p.N || token >= p.T || (p.epilogue != EPI_SWIGLU && p.epilogue != EPI_STORE)) {
+        emit16(p, r, token, f0);
+        emit16(p, r + 16, token, f0 + 16);
+        return;
+    }
+    if (p.epilogue == EPI_SWIGLU) {
+        float a[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const int g = (j & 7) + (j >> 3) * 16;
+            a[j] = gated_unit(p, __uint_as_float(r[g]), __uint_as_float(r[g + 8]));
+        }
+        const int64_t at = (int64_t)token * p.ldo + (f0 >> 1);
+        uint32_t o[16];
+        if (p.out_f32) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(a[j]);
+            store_32((float*)p.out + at, o);
+            store_32((float*)p.out + at + 8, o + 8);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = pack_bf16(a[2 * j], a[2 * j + 1]);
+            store_32((__nv_bfloat16*)p.out + at, o);
+        }
+        return;
+    }
+    const int64_t at = (int64_t)token * p.ldo + f0;
+    if (p.out_f32) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) store_32((float*)p.out + at + 8 * q, r + 8 * q);
+    } else {
+        uint32_t o[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+        store_32((__nv_bfloat16*)p.out + at, o);
+        store_32((__nv_bfloat16*)p.out + at + 16, o + 8);
+    }
+}
+
+// One epilogue warp's share of a tile of the many-token kernels: its 32 lanes of tensor memory (tokens), half of the tile's BN
+// columns, 32 at a time; the next 32 are on their way while these leave. `handed_back` is called when the last of them are in
+// registers. What the gated epilogue costs decides whether the next tile's products hide it: a 256 x 256 tile of K = 1024 is
+// 4.4 us of tensor-core time, and with four warps, a division an output and 16-byte stores the epilogue took 15 us. Measured on
+// B200 with the gated epilogue (us, before -> now): 8,192 tokens N 13312 K 1024 352 -> 196 (1.14 PFLOP/s; 167 storing the product
+// as it is, the vendor's product 165), 8,192 x 16384 x 2048 452 -> 390, 2,048 x 16384 x 2048 124 -> 104.
+template <int BN, typename F>
+__device__ __forceinline__ void drain_half(const GemmTcParams& p, uint32_t acc, int half, int token, bool live, int f0, F handed_back) {
+    constexpr int kParts = BN / 64;
+    uint32_t r[2][32];
+    tmem_ask32(acc + (uint32_t)(half * (BN / 2)), r[0]);
+#pragma unroll
+    for (int c = 0; c < kParts; ++c) {
+        tmem_landed(r[c & 1]);
+        if (c + 1 < kParts) tmem_ask32(acc + (uint32_t)(half * (BN / 2) + (c + 1) * 32), r[(c + 1) & 1]);
+        else handed_back();
+        if (live) emit32(p, r[c & 1], token, f0 + half * (BN / 2) + c * 32);
     }
 }
 
@@ -341,7 +411,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // one token and stores 16 bytes at a time. Two accumulators in tensor memory: while the epilogue warps drain
 // tile i, the MMA warp already works on tile i + 1. The stage ring runs on across tiles.
 template <int BN, int STAGES>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kManyThreads, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                           const GemmTcParams p, int tiles_tok, int tiles_f) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -366,7 +436,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gr
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&bar_acc_full[b]), 1);
-            mbar_init(smem_u32(&bar_acc_empty[b]), 4);           // one arrival per epilogue warp
+            mbar_init(smem_u32(&bar_acc_empty[b]), 8);           // one arrival per epilogue warp
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -431,16 +501,12 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gr
             if (!mbar_wait(smem_u32(&bar_acc_full[buf]), (lt >> 1) & 1, abort_p)) break;
             tcgen05_fence_after();
             const int token = tile_tok * BM + quarter * 32 + lane;
-#pragma unroll 1
-            for (int c = 0; c < BN; c += 32) {
-                uint32_t r[32];
-                tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c), r);
-                emit16(p, r, token, tile_f * BN + c);
-                emit16(p, r + 16, token, tile_f * BN + c + 16);
-            }
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[buf]));
+            drain_half<BN>(p, tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN), (warp - 2) >> 2, token, true,
+                           tile_f * BN, [&] {
+                               tcgen05_fence_before();
+                               __syncwarp();
+                               if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[buf]));
+                           });
         }
         tcgen05_fence_before();
     }
@@ -532,7 +598,7 @@ constexpr int kPairTile = 256;                               // weight rows and 
 constexpr int kPairStageBytes = 2 * BM * BK * 2;             // per CTA: 128 weight rows and 128 tokens, 64 k each
 
 template <int STAGES>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kManyThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                     const GemmTcParams p, int tiles_tok, int tiles_f) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -540,7 +606,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     __shared__ __align__(8) uint64_t bar_full[STAGES];       // used in the leader only
     __shared__ __align__(8) uint64_t bar_empty[STAGES];      // one set per CTA, signalled by the leader's commits
     __shared__ __align__(8) uint64_t bar_acc_full[2];        // one set per CTA
-    __shared__ __align__(8) uint64_t bar_acc_empty[2];       // used in the leader only: 8 epilogue warps arrive
+    __shared__ __align__(8) uint64_t bar_acc_empty[2];       // used in the leader only: 16 epilogue warps arrive
     __shared__ uint32_t tmem_base;
     __shared__ int abort_flag;
 
@@ -560,7 +626,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&bar_acc_full[b]), 1);
-            mbar_init(smem_u32(&bar_acc_empty[b]), 8);
+            mbar_init(smem_u32(&bar_acc_empty[b]), 16);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -626,16 +692,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             if (!mbar_wait_cluster(smem_u32(&bar_acc_full[buf]), (lt >> 1) & 1, abort_p)) break;
             tcgen05_fence_after();
             const int token = tile_tok * kPairTile + (int)rank * BM + quarter * 32 + lane;
-#pragma unroll 1
-            for (int c = 0; c < kPairTile; c += 32) {
-                uint32_t r[32];
-                tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * kPairTile + c), r);
-                emit16(p, r, token, tile_f * kPairTile + c);
-                emit16(p, r + 16, token, tile_f * kPairTile + c + 16);
-            }
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&bar_acc_empty[buf]), 0));
+            drain_half<kPairTile>(p, tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * kPairTile), (warp - 2) >> 2, token,
+                                  true, tile_f * kPairTile, [&] {
+                                      tcgen05_fence_before();
+                                      __syncwarp();
+                                      if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&bar_acc_empty[buf]), 0));
+                                  });
         }
         tcgen05_fence_before();
     }
@@ -673,7 +735,7 @@ int launch_persistent(const CUtensorMap& mx, const CUtensorMap& mw, const GemmTc
     }
     const int tiles_tok = ceil_div_i(p.T, BM), tiles_f = ceil_div_i(p.N, BN);
     const int grid = tiles_tok * tiles_f < sms ? tiles_tok * tiles_f : sms;
-    return xs_launch(gemm_tc_persistent_kernel<BN, STAGES>, dim3(grid), dim3(kThreads), smem, stream, mx, mw, p, tiles_tok,
+    return xs_launch(gemm_tc_persistent_kernel<BN, STAGES>, dim3(grid), dim3(kManyThreads), smem, stream, mx, mw, p, tiles_tok,
                      tiles_f) == cudaSuccess ? 0 : -1;
 }
 
@@ -686,7 +748,7 @@ int launch_persistent(const CUtensorMap& mx, const CUtensorMap& mw, const GemmTc
 // tiles. A weight box that reaches past an expert's last row reads the next expert's (or zeros at the end): those
 // columns are not stored.
 template <int BN, int STAGES>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kManyThreads, 1)
 gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                        const GemmTcParams p, const int32_t* __restrict__ meta, int tiles_f, int w_rows) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -710,7 +772,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&bar_acc_full[b]), 1);
-            mbar_init(smem_u32(&bar_acc_empty[b]), 4);
+            mbar_init(smem_u32(&bar_acc_empty[b]), 8);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -779,18 +841,12 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
             tcgen05_fence_after();
             const int local = quarter * 32 + lane;
             const int token = row0 + local;
-#pragma unroll 1
-            for (int c = 0; c < BN; c += 32) {
-                uint32_t r[32];
-                tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c), r);
-                if (local < rows) {
-                    emit16(p, r, token, tile_f * BN + c);
-                    emit16(p, r + 16, token, tile_f * BN + c + 16);
-                }
-            }
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[buf]));
+            drain_half<BN>(p, tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN), (warp - 2) >> 2, token, local < rows,
+                           tile_f * BN, [&] {
+                               tcgen05_fence_before();
+                               __syncwarp();
+                               if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[buf]));
+                           });
         }
         tcgen05_fence_before();
     }
@@ -817,7 +873,7 @@ int launch_grouped(const CUtensorMap& mx, const CUtensorMap& mw, const GemmTcPar
     const int tiles_f = ceil_div_i(w_rows, BN);
     const int64_t most = (int64_t)max_m_tiles * tiles_f;
     const int grid = most < sms ? (int)most : sms;
-    return xs_launch(gemm_tc_grouped_kernel<BN, STAGES>, dim3(grid), dim3(kThreads), smem, stream, mx, mw, p, meta, tiles_f,
+    return xs_launch(gemm_tc_grouped_kernel<BN, STAGES>, dim3(grid), dim3(kManyThreads), smem, stream, mx, mw, p, meta, tiles_f,
                      w_rows) == cudaSuccess ? 0 : -1;
 }
 
@@ -837,7 +893,7 @@ int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmTcParams
         // how many pairs can run at one time: SMs pair up inside a GPC only
         cudaLaunchConfig_t probe = {};
         probe.gridDim = dim3(2 * (sms / 2));
-        probe.blockDim = dim3(kThreads);
+        probe.blockDim = dim3(kManyThreads);
         probe.dynamicSmemBytes = smem;
         cudaLaunchAttribute a[1];
         a[0].id = cudaLaunchAttributeClusterDimension;
@@ -855,7 +911,7 @@ int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmTcParams
     const int pairs = tiles_tok * tiles_f < max_pairs ? tiles_tok * tiles_f : max_pairs;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(kManyThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -946,7 +1002,7 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* o
         // many tokens: the tokens on the M side, 128 or 256 weight rows on the N side; pairs of CTAs beyond 128 tokens
         XS_REQUIRE(ksplit == 1, "gemm (tcgen05): K slices are for at most 64 tokens");
         const int esz = p.out_f32 ? 4 : 2;
-        p.vec = ((uintptr_t)out % 16 == 0) && ((ldo * esz) % 16 == 0);
+        p.vec = (uintptr_t)out % 32 == 0 && (ldo * esz) % 32 == 0 ? 2 : (uintptr_t)out % 16 == 0 && (ldo * esz) % 16 == 0;
         const bool pair = T > 128 && g_pair;
         const int box_w = (pair || N <= 128) ? 128 : 256;
         XS_REQUIRE(make_map(&mx, x, T, K, ldx, BM), "gemm (tcgen05): the input's tensor map could not be made");
@@ -1010,7 +1066,7 @@ XS_API int xs_gemm_tc_grouped(const void* x, const void* w, void* out, int out_d
     // (the gated epilogue's activation: limit 0 is silu(gate) * up, limit > 0 the clamped unit's)
     p.glu_limit = glu_limit; p.glu_alpha = glu_alpha; p.glu_shift = glu_shift; p.glu_act = 0;
     const int esz = p.out_f32 ? 4 : 2;
-    p.vec = ((uintptr_t)out % 16 == 0) && ((ldo * esz) % 16 == 0);
+    p.vec = (uintptr_t)out % 32 == 0 && (ldo * esz) % 32 == 0 ? 2 : (uintptr_t)out % 16 == 0 && (ldo * esz) % 16 == 0;
     alignas(64) CUtensorMap mw, mx;
     const int box_w = N <= 128 ? 128 : 256;
     XS_REQUIRE(make_map(&mx, x, rows_cap, K, ldx, BM), "gemm (tcgen05, grouped): the input's tensor map could not be made");
