@@ -1,5 +1,6 @@
-"""Products and attention in float32, each alone against float64, at the edges of their tiles, stages and dispatch lines. Limits:
-a float32 sum of K products in any order is within about sqrt(K) / 2 roundings of 2^-24 of sqrt(sum of squares)."""
+"""The float32 products and attention, the many-token product's stores and the experts' product for few tokens, each alone against
+float64, at the edges of their tiles, stages and dispatch lines. Limits: a float32 sum of K products in any order is within
+about sqrt(K) / 2 roundings of 2^-24 of sqrt(sum of squares); outputs rounded to bfloat16 are within 2^-9 of their size."""
 import math
 
 import pytest
@@ -8,6 +9,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 DEV = "cuda"
+BF = torch.bfloat16
 
 
 def ops():
@@ -92,3 +94,103 @@ def test_float32_attention(H, G, D, DV, planes, window, keep, plus, cap, lens):
                 w = torch.softmax(z, 0)
             ref[t, h] = w @ v * torch.sigmoid(gate[t, h].double())
     assert gap(out, ref) <= 4e-6      # (scores of a few units: 2^-24 of them through the exponential, on top of the sums)
+
+
+# --------------------------------------------------------------------------- tcgen05 product, many tokens: the store paths
+@pytest.mark.parametrize("T,N", [(65, 48), (128, 272), (129, 256), (300, 528), (1000, 80)])
+@pytest.mark.parametrize("pad", [0, 8, 1])
+@pytest.mark.parametrize("form", ["store", "store32", "swiglu", "swiglu32", "clamped"])
+def test_many_token_product_stores(T, N, pad, form):
+    """Rows of the output on 32-byte, 16-byte and odd boundaries, tiles that end inside 32 columns."""
+    K = 72
+    x, w = torch.randn(T, K, device=DEV).to(BF), torch.randn(N, K, device=DEV).to(BF)
+    gated = not form.startswith("store")
+    cols, dtype = N // 2 if gated else N, torch.float32 if form.endswith("32") else BF
+    out = torch.full((T, (cols + 15) // 16 * 16 + pad), 7.0, device=DEV, dtype=dtype)
+    if form == "clamped":
+        ops().gemm_tc_clamped(x, w, out[:, :cols], 1.5, 1.702, 1.0)
+    else:
+        ops().gemm_tc(x, w, out[:, :cols], epilogue=ops().EPI_SWIGLU if gated else ops().EPI_STORE)
+    ref = x.double() @ w.double().T
+    if gated:
+        g, u = ref.view(T, N // 16, 2, 8).unbind(2)
+        g, u = g.reshape(T, cols), u.reshape(T, cols)
+        if form == "clamped":
+            g, u = g.clamp(max=1.5), u.clamp(-1.5, 1.5)
+            ref = g * torch.sigmoid(1.702 * g) * (u + 1.0)
+        else:
+            ref = g * torch.sigmoid(g) * u
+    # (the exponential's and the reciprocal's few units in the last place on top of the sums)
+    assert gap(out[:, :cols], ref) <= (2.0 ** -8 if dtype == BF else f32_limit(K) + 2.0 ** -20)
+    assert bool((out[:, cols:] == 7.0).all())
+
+
+def test_gated_epilogue_far_gates():
+    """Gates where the exponential is zero, huge or infinite."""
+    gates = torch.tensor([0.0, -80.0, -88.0, -88.6, -100.0, -3e4, 80.0, 100.0, 3e4], device=DEV)
+    T, K = 130, 16
+    x = torch.zeros(T, K, device=DEV, dtype=BF)
+    x[:, 0] = gates[torch.arange(T, device=DEV) % len(gates)].to(BF)
+    x[:, 1] = 3.0
+    w = torch.zeros(16, K, device=DEV, dtype=BF)
+    w[:8, 0], w[8:, 1] = 1.0, 1.0
+    out = torch.empty(T, 8, device=DEV)
+    ops().gemm_tc(x, w, out, epilogue=ops().EPI_SWIGLU)
+    g = x[:, :1].double()
+    assert gap(out, (g * torch.sigmoid(g) * 3.0).expand(T, 8)) <= 2.0 ** -20
+    small = g[:, 0] < -10
+    assert ((out[small].double() - (g * torch.sigmoid(g) * 3.0)[small]).abs() <= 1e-30).all()
+
+
+# ------------------------------------------------------------------------------------------- few tokens' experts
+@pytest.mark.parametrize("T,top,E,F,H", [(1, 1, 1, 8, 8), (1, 4, 16, 1024, 2048), (7, 3, 5, 24, 40), (8, 2, 3, 40, 264), (9, 1, 1, 16, 512),
+                                         (16, 4, 6, 56, 96), (17, 2, 4, 48, 1032), (32, 5, 7, 72, 328)])
+@pytest.mark.parametrize("act", ["silu", "clamped", "relu_squared"])
+def test_experts_of_few_tokens(T, top, E, F, H, act):
+    top = min(top, E)
+    x = torch.randn(T, H + 8, device=DEV).to(BF)[:, :H]
+    ids = torch.stack([torch.randperm(E, device=DEV)[:top] for _ in range(T)]).to(torch.int32).reshape(-1)
+    if T * top > 3:
+        ids[2] = -1
+    gate, up = (torch.randn(E, F, H, device=DEV).to(BF) * H ** -0.5 for _ in range(2))
+    down = (torch.randn(E, H, F, device=DEV) * F ** -0.5).to(BF)
+    glu = act != "relu_squared"
+    w = torch.stack([gate.view(E, F // 8, 8, H), up.view(E, F // 8, 8, H)], 2).reshape(E, 2 * F, H).contiguous() if glu else up.contiguous()
+    hidden = torch.zeros(T * top, F, device=DEV, dtype=BF)
+    clamp = (1.0, 1.702, 1.0) if act == "clamped" else None
+    ops().moe_few_rows(x, top, w, hidden, ids, T, glu=glu, clamp=clamp, relu_squared=not glu)
+    out = torch.zeros(T * top, H, device=DEV, dtype=BF)
+    ops().moe_few_rows(hidden, 1, down, out, ids, T, glu=False)
+    for i in range(T * top):
+        e = int(ids[i])
+        if e < 0:
+            assert not hidden[i].any() and not out[i].any()
+            continue
+        u = up[e].double() @ x[i // top].double()
+        g = gate[e].double() @ x[i // top].double()
+        if act == "silu":
+            ref = g * torch.sigmoid(g) * u
+        elif act == "clamped":
+            g, u = g.clamp(max=1.0), u.clamp(-1.0, 1.0)
+            ref = g * torch.sigmoid(1.702 * g) * (u + 1.0)
+        else:
+            ref = u.clamp(min=0.0) ** 2
+        assert gap(hidden[i], ref) <= 2.0 ** -8 and gap(out[i], down[e].double() @ hidden[i].double()) <= 2.0 ** -8
+    wts = torch.rand(T * top, device=DEV)
+    y = torch.empty(T, H, device=DEV, dtype=BF)
+    ops().moe_combine(out, ids, wts, y, top, in_place=True, passed=x)
+    rows = torch.where((ids >= 0)[:, None], out.double(), x.double().repeat_interleave(top, 0))
+    assert gap(y, (rows * wts.double()[:, None]).view(T, top, H).sum(1)) <= 2.0 ** -8
+
+
+def test_experts_rows_do_not_depend_on_the_step():
+    E, F, H, top = 6, 64, 256, 2
+    x = torch.randn(8, H, device=DEV).to(BF)
+    ids = torch.randint(0, E, (8,), device=DEV)
+    ids = torch.stack([ids, (ids + 1) % E], 1).to(torch.int32).reshape(-1)
+    w = torch.randn(E, F, H, device=DEV).to(BF)
+    whole, one = torch.empty(16, F, device=DEV, dtype=BF), torch.empty(2, F, device=DEV, dtype=BF)
+    ops().moe_few_rows(x, top, w, whole, ids, 8, glu=False)
+    for t in range(8):
+        ops().moe_few_rows(x[t:t + 1], top, w, one, ids[2 * t:2 * t + 2].contiguous(), 1, glu=False)
+        assert torch.equal(one, whole[2 * t:2 * t + 2])

@@ -504,7 +504,7 @@ template <typename TI, typename TO>
 __global__ void moe_combine_kernel(const TI* __restrict__ rows_out, const int32_t* __restrict__ place,
                                    const float* __restrict__ wts, TO* __restrict__ y, int H, int top,
                                    const TI* __restrict__ shared, const float* __restrict__ shared_gate, int ld_gate,
-                                   const TI* __restrict__ passed, int64_t ld_passed) {
+                                   const TI* __restrict__ passed, int64_t ld_passed, int in_place) {
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x;
@@ -514,12 +514,69 @@ __global__ void moe_combine_kernel(const TI* __restrict__ rows_out, const int32_
         float v = shared == nullptr ? 0.0f : sg * to_f32(shared[(int64_t)t * H + c]);
         for (int k = 0; k < top; ++k) {
             // (a choice without a place is an expert that hands its input through: `passed` holds the tokens' inputs)
-            const int pl = place[(int64_t)t * top + k];
+            int pl = place[(int64_t)t * top + k];
+            if (in_place && pl >= 0) pl = t * top + k;      // (`place` holds the experts: rows stand where the router left them)
             const float r = pl >= 0 ? to_f32(rows_out[(int64_t)pl * H + c]) : passed != nullptr ? to_f32(passed[(int64_t)t * ld_passed + c]) : 0.0f;
             v = fmaf(wts[(int64_t)t * top + k], r, v);
         }
         y[(int64_t)t * H + c] = from_f32<TO>(v);
     }
+}
+
+// The same eight columns a thread (H a multiple of 8, 16-byte rows): the rows' loads are 16 bytes and those of up to four
+// choices are in flight together; the sums' order is the same.
+__global__ void moe_combine_bf16x8_kernel(const __nv_bfloat16* __restrict__ rows_out, const int32_t* __restrict__ place,
+                                          const float* __restrict__ wts, __nv_bfloat16* __restrict__ y, int T, int H, int top,
+                                          const __nv_bfloat16* __restrict__ shared, const float* __restrict__ shared_gate, int ld_gate,
+                                          const __nv_bfloat16* __restrict__ passed, int64_t ld_passed, int in_place) {
+    pdl_launch_dependents();
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = (int)(i / (H >> 3)), c = (int)(i % (H >> 3)) * 8;
+    pdl_wait();
+    if (t >= T) return;
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+    float v[8];
+    {
+        const float sg = shared == nullptr ? 0.0f : shared_gate == nullptr ? 1.0f : sigmoid_f(shared_gate[(int64_t)t * ld_gate]);
+        const uint4 raw = shared == nullptr ? none : *reinterpret_cast<const uint4*>(shared + (int64_t)t * H + c);
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 f = __bfloat1622float2(h[j]);
+            v[2 * j] = shared == nullptr ? 0.0f : sg * f.x;
+            v[2 * j + 1] = shared == nullptr ? 0.0f : sg * f.y;
+        }
+    }
+    for (int k0 = 0; k0 < top; k0 += 4) {
+        uint4 raw[4];
+        float w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool there = k0 + k < top;
+            const int row = t * top + k0 + k;
+            int pl = there ? place[row] : -1;
+            if (in_place && pl >= 0) pl = row;             // (`place` holds the experts: rows stand where the router left them)
+            w[k] = there ? wts[row] : 0.0f;
+            raw[k] = pl >= 0 ? *reinterpret_cast<const uint4*>(rows_out + (int64_t)pl * H + c)
+                     : there && passed != nullptr ? *reinterpret_cast<const uint4*>(passed + (int64_t)t * ld_passed + c) : none;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k0 + k >= top) break;
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[k]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 f = __bfloat1622float2(h[j]);
+                v[2 * j] = fmaf(w[k], f.x, v[2 * j]);
+                v[2 * j + 1] = fmaf(w[k], f.y, v[2 * j + 1]);
+            }
+        }
+    }
+    uint4 o;
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+    *reinterpret_cast<uint4*>(y + (int64_t)t * H + c) = o;
 }
 
 }  // namespace
@@ -668,14 +725,22 @@ XS_API int xs_moe_gather(const void* x, int64_t ldx, const int32_t* source, int 
 }
 
 XS_API int xs_moe_combine(const void* rows_out, const int32_t* place, const float* wts, void* y, int T, int H, int top,
-                          const void* shared, const float* shared_gate, int ld_gate, const void* passed, int64_t ld_passed, int dtype,
-                          cudaStream_t stream) {
+                          const void* shared, const float* shared_gate, int ld_gate, const void* passed, int64_t ld_passed, int in_place,
+                          int dtype, cudaStream_t stream) {
     if (T == 0) return 0;
     XS_REQUIRE(T > 0 && H > 0 && top > 0, "moe_combine: %d tokens of %d, top %d", T, H, top);
+    if (dtype == XS_BF16 && H % 8 == 0 && ld_passed % 8 == 0 &&
+        ((uintptr_t)rows_out | (uintptr_t)y | (uintptr_t)shared | (uintptr_t)passed) % 16 == 0) {
+        xs_launch(moe_combine_bf16x8_kernel, dim3(ceil_div_i((int64_t)T * (H / 8), 128)), dim3(128), 0, stream, (const __nv_bfloat16*)rows_out,
+                  place, wts, (__nv_bfloat16*)y, T, H, top, (const __nv_bfloat16*)shared, shared_gate, ld_gate, (const __nv_bfloat16*)passed,
+                  ld_passed, in_place);
+        XS_LAUNCH_CHECK("moe_combine");
+        return 0;
+    }
     XS_DISPATCH_DTYPE(dtype, TT,
                       xs_launch(moe_combine_kernel<TT, TT>, dim3(T), dim3(H >= 1024 ? 256 : 128), 0, stream,
                                 (const TT*)rows_out, place, wts, (TT*)y, H, top, (const TT*)shared, shared_gate, ld_gate,
-                                (const TT*)passed, ld_passed));
+                                (const TT*)passed, ld_passed, in_place));
     XS_LAUNCH_CHECK("moe_combine");
     return 0;
 }

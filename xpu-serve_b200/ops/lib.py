@@ -71,7 +71,8 @@ def _signatures(lib) -> None:
         "xs_moe_gather": [P, L, P, I, P, I, I, P],
         "xs_gemm_tc_grouped": [P, P, P, I, I, P, I, I, I, I, I, L, L, F, F, F, P, P],
         "xs_moe_gemm": [P, L, P, P, L, P, I, P, I, I, I, I, F, F, F, I, I, P],
-        "xs_moe_combine": [P, P, P, P, I, I, I, P, P, I, P, L, I, P],
+        "xs_moe_combine": [P, P, P, P, I, I, I, P, P, I, P, L, I, I, P],
+        "xs_moe_few_rows": [P, L, I, P, P, L, P, I, I, I, I, I, I, F, F, F, P],
         "xs_relu_squared": [P, P, I, L, P],
         "xs_embed_pair": [P, P, I, P, P, P, P, P, P, P, P, P, I, I, F, I, ctypes.c_longlong, ctypes.c_longlong, F, P],
         "xs_mlstm_scan": [P, L, I, I, I, P, L, P, P, P, P, P, P, P, I, I, I, I, F, F, I, P, P, I, P, P, P],
@@ -1069,11 +1070,12 @@ def moe_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, meta: torch.Te
 
 def moe_combine(rows_out: torch.Tensor, place: torch.Tensor, wts: torch.Tensor, y: torch.Tensor, top: int,
                 shared: Optional[torch.Tensor] = None, shared_gate: Optional[torch.Tensor] = None,
-                passed: Optional[torch.Tensor] = None) -> None:
+                passed: Optional[torch.Tensor] = None, in_place: bool = False) -> None:
     """y[t] = sum_k wts[t, k] * rows_out[place[t, k]], summed in float32 in the order of k. `shared` [T, H] (a unit that
     every token uses) starts the sum, times sigmoid(shared_gate[t, 0]) when `shared_gate` (float32, one row a token whose
     first column is the gate's logit) is given. `passed` [T, H] (the tokens' inputs): a choice whose place is -1 adds its
-    weight times the token's input (an expert that hands its input through)."""
+    weight times the token's input (an expert that hands its input through). `in_place`: the rows stand where the router
+    left them (row t * top + k), and `place` holds the router's ids, of which only a -1 says something."""
     _need(rows_out, "expert outputs", y.dtype); _need(y, "y")
     T, H = y.shape
     ld_gate = 0
@@ -1089,7 +1091,30 @@ def moe_combine(rows_out: torch.Tensor, place: torch.Tensor, wts: torch.Tensor, 
             ld_gate = shared_gate.stride(0)
     _check(load().xs_moe_combine(rows_out.data_ptr(), place.data_ptr(), wts.data_ptr(), y.data_ptr(), T, H, int(top),
                                  _ptr(shared), _ptr(shared_gate) if shared is not None else None, ld_gate, _ptr(passed),
-                                 0 if passed is None else passed.stride(0), _code(y), _stream()))
+                                 0 if passed is None else passed.stride(0), int(in_place), _code(y), _stream()))
+
+
+MOE_FEW_TOKENS = 32      # the most tokens `moe_few_rows` takes (an expert then has at most as many rows)
+
+
+def moe_few_rows(x: torch.Tensor, share: int, w: torch.Tensor, out: torch.Tensor, ids: torch.Tensor, tokens: int, glu: bool,
+                 clamp=None, relu_squared: bool = False) -> None:
+    """out[i] = w[ids[i]] . x[i // share] for the rows i of a step's choices in the router's own order (rows whose id is -1 are
+    left alone), `tokens` at most MOE_FEW_TOKENS. w, `glu`, `clamp` and `relu_squared` as in gemm_tc_grouped."""
+    limit, alpha, shift = (0.0, 1.0, 0.0) if clamp is None else clamp
+    if glu and relu_squared:
+        raise KernelError("moe_few_rows: one activation at a time")
+    _need(w, "expert weights", torch.bfloat16); _need(ids, "ids", torch.int32)
+    E, N, K = w.shape
+    rows = ids.numel()
+    for t, name in ((x, "x"), (out, "out")):
+        if not t.is_cuda or t.dtype != torch.bfloat16 or t.dim() != 2 or t.stride(1) != 1:
+            raise KernelError(f"moe_few_rows: {name} must be a bfloat16 CUDA matrix with contiguous rows")
+    if x.shape[1] != K or x.shape[0] * share < rows or out.shape[0] < rows or out.shape[1] != (N // 2 if glu else N):
+        raise KernelError(f"moe_few_rows: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}, {rows} rows")
+    _check(load().xs_moe_few_rows(x.data_ptr(), x.stride(0), int(share), w.data_ptr(), out.data_ptr(), out.stride(0), ids.data_ptr(),
+                                  rows, int(tokens), E, N, K, 1 if glu else 2 if relu_squared else 0, float(limit), float(alpha),
+                                  float(shift), _stream()))
 
 
 def relu_squared(x: torch.Tensor, out: torch.Tensor) -> None:

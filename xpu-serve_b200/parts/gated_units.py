@@ -197,6 +197,14 @@ class RoutedExperts(FeedForward):
             ops.moe_route(logits, s.top, ids, wts, experts=s.experts, scale=s.route_scale)
         out = ws.get("ffn_out", (T, s.hidden), rt.act_dtype)
         passed = {"passed": y} if self.identity else {}       # (choices that stand for the token's input itself)
+        if self.tensor_cores and T <= ops.MOE_FEW_TOKENS:
+            # few tokens: the products find each expert's rows in the router's ids, which stay in their order (csrc/experts_few.cu)
+            act = ws.get("moe_act_few", (n, s.intermediate), rt.act_dtype)
+            ops.moe_few_rows(y, s.top, self.w_gate_up, act, ids, T, glu=self.gated, clamp=self.clamp, relu_squared=not self.gated)
+            rows_out = ws.get("moe_rows_few", (n, s.hidden), rt.act_dtype)
+            ops.moe_few_rows(act, 1, self.w_down, rows_out, ids, T, glu=False)
+            ops.moe_combine(rows_out, ids, wts, out, s.top, shared, shared_gate, in_place=True, **passed)
+            return out
         if self.tensor_cores:
             # every expert's rows padded to tiles of 128: gather, two tcgen05 products over the plan's tiles, combine
             tiles = ops.moe_max_tiles_of(n, s.experts, 128)
