@@ -1,5 +1,5 @@
-"""The float32 products and attention, the many-token product's stores and the experts' product for few tokens, each alone against
-float64, at the edges of their tiles, stages and dispatch lines. Limits: a float32 sum of K products in any order is within
+"""The float32 products and attention, the many-token product's stores, the experts' product for few tokens and kernels of the
+recurrent and latent layers, each alone against float64, at the edges of their tiles, stages and dispatch lines. Limits: a float32 sum of K products in any order is within
 about sqrt(K) / 2 roundings of 2^-24 of sqrt(sum of squares); outputs rounded to bfloat16 are within 2^-9 of their size."""
 import math
 
@@ -194,3 +194,54 @@ def test_experts_rows_do_not_depend_on_the_step():
     for t in range(8):
         ops().moe_few_rows(x[t:t + 1], top, w, one, ids[2 * t:2 * t + 2].contiguous(), 1, glu=False)
         assert torch.equal(one, whole[2 * t:2 * t + 2])
+
+
+# ------------------------------------------------------------------------- kernels of the recurrent and latent layers
+@pytest.mark.parametrize("B,M,N,K", [(1, 1, 1, 8), (16, 8, 512, 128), (3, 9, 33, 520), (2, 16, 31, 1032), (4, 5, 100, 24)])
+def test_batched_product_of_few_rows(B, M, N, K):
+    x = torch.randn(M, B, K + 8, device=DEV).to(BF).transpose(0, 1)[:, :, :K]
+    w = torch.randn(B, N, K + 16, device=DEV).to(BF)[:, :, :K]
+    out = torch.empty(M, B, N, device=DEV, dtype=BF).transpose(0, 1)
+    ops().gemm_batched(x, w, out)
+    assert gap(out, x.double() @ w.double().transpose(1, 2)) <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("groups,part", [(2, 4), (3, 100), (16, 128), (5, 132), (8, 512), (2, 516), (2, 1024)])
+@pytest.mark.parametrize("act", [None, 0, 1])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_grouped_norm(groups, part, act, dtype):
+    T, W, eps = 5, groups * part, 1e-5
+    x, w = torch.randn(T, W, device=DEV), torch.rand(W, device=DEV) + 0.5
+    y = torch.empty(T, W, device=DEV, dtype=dtype)
+    gate = torch.randn(T, W + 3, device=DEV).to(dtype)[:, 3:] if act is not None else None
+    ops()._check(ops().load().xs_grouped_rmsnorm(x.data_ptr(), w.data_ptr(), y.data_ptr(), W, ops()._code(y), T, W, groups, eps,
+                                                 ops()._ptr(gate), 0 if gate is None else gate.stride(0), act or 0, ops()._stream()))
+    v = x.double().view(T, groups, part)
+    ref = (v * torch.rsqrt((v * v).mean(-1, keepdim=True) + eps)).view(T, W) * w.double()
+    if gate is not None:
+        z = gate.double()
+        ref = ref * torch.sigmoid(z) * (z if act == 1 else 1.0)
+    assert gap(y, ref) <= (2.0 ** -8 if dtype == BF else 2e-6)
+
+
+@pytest.mark.parametrize("heads,P,N,G,seqs", [(4, 4, 1, 2, 1), (6, 64, 128, 3, 8), (2, 20, 37, 1, 3), (3, 132, 300, 3, 2), (2, 1024, 16, 1, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_mamba2_step(heads, P, N, G, seqs, dtype):
+    inner = heads * P
+    C = inner + 2 * G * N
+    r = lambda *s: torch.randn(*s, device=DEV)                                     # noqa: E731
+    xbc, proj = r(seqs, C).to(dtype), r(seqs, inner + C + heads).to(dtype)
+    bias, a_log, skip, state0 = r(heads), r(heads) * 0.5, r(heads), r(seqs + 2, heads, N, P)
+    slots = torch.randperm(seqs + 2, device=DEV)[:seqs].to(torch.int32)
+    cu = torch.arange(seqs + 1, dtype=torch.int32, device=DEV)
+    state, y = state0.clone(), torch.empty(seqs, inner, device=DEV)
+    ops().mamba2_scan(xbc, proj, inner + C, bias, a_log, skip, state, cu, slots, y, heads, P, N, G, single=True)
+    x = xbc.double()[:, :inner].view(seqs, heads, P)
+    Bm, Cm = (m.view(seqs, G, N).repeat_interleave(heads // G, 1) for m in xbc.double()[:, inner:].split(G * N, 1))
+    dt = torch.nn.functional.softplus(proj.double()[:, inner + C:] + bias.double())
+    s = state0[slots.long()].double() * torch.exp(-torch.exp(a_log.double()) * dt)[..., None, None] + (dt[..., None] * Bm)[..., None] * x[:, :, None]
+    want = ((s * Cm[..., None]).sum(2) + skip.double()[:, None] * x).reshape(seqs, inner)
+    want = want * torch.nn.functional.silu(proj.double()[:, :inner])
+    assert gap(y, want) <= 4e-6 and gap(state[slots.long()], s) <= 2e-6
+    rest = torch.tensor([i for i in range(seqs + 2) if i not in set(slots.tolist())], device=DEV)
+    assert torch.equal(state[rest], state0[rest])

@@ -16,6 +16,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "few_rows.cuh"
 
 namespace {
 
@@ -357,6 +358,43 @@ gemm_batched_few_rows_kernel(const T* __restrict__ x, int64_t ldx, int64_t sx, c
     }
 }
 
+// The same on tensor cores (bfloat16, K a multiple of 8, rows in 16-byte pieces): 32 weight rows of one batch a CTA, whose warps
+// share K and add up in shared memory in their order. Measured on B200 (16 heads, 8 rows: N 512 K 128, and N 128 K 512): 3.8 and
+// 4.3 us; the kernel above 13.6 and 12.9, which reads 2 bytes of a weight a lane at a time behind a pass of all of x through shared
+// memory.
+template <int NT>
+__global__ void __launch_bounds__(kFewWarps * 32)
+gemm_batched_few_rows_mma_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int64_t sx, const __nv_bfloat16* __restrict__ w, int64_t ldw,
+                                 int64_t sw, __nv_bfloat16* __restrict__ out, int64_t ldo, int64_t so, int M, int N, int K) {
+    __shared__ float sums[kFewWarps][2 * NT * 4][32];
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, piece = (lane & 3) * 8, r = lane >> 2;
+    const int n0 = blockIdx.x * kFewRows;
+    const __nv_bfloat16 *wr[4], *xr[NT];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) wr[q] = w + (int64_t)blockIdx.y * sw + (int64_t)min(n0 + r + 8 * q, N - 1) * ldw + piece;
+#pragma unroll
+    for (int t = 0; t < NT; ++t) xr[t] = x + (int64_t)blockIdx.y * sx + (int64_t)min(8 * t + r, M - 1) * ldx + piece;
+    float acc[2][NT][4] = {};
+    pdl_wait();
+    few_rows_multiply<NT>(wr, xr, K, piece, warp, acc);
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sums[warp][(m * NT + t) * 4 + j][lane] = acc[m][t][j];
+    __syncthreads();
+    for (int item = threadIdx.x; item < 2 * NT * 4 * 32; item += kFewWarps * 32) {
+        const int l = item & 31, e = item >> 5, j = e & 3, t = (e >> 2) % NT, m = (e >> 2) / NT;
+        const int row = 8 * t + (l & 3) * 2 + (j & 1), n = n0 + 16 * m + (l >> 2) + 8 * (j >> 1);
+        float v = 0.0f;
+#pragma unroll
+        for (int k = 0; k < kFewWarps; ++k) v += sums[k][e][l];
+        if (row < M && n < N) out[(int64_t)blockIdx.y * so + (int64_t)row * ldo + n] = __float2bfloat16_rn(v);
+    }
+}
+
 }  // namespace
 
 XS_API int xs_latent_prepare(const void* down, int64_t ld_down, const void* q, int64_t ld_q, const float* norm_w,
@@ -410,6 +448,14 @@ XS_API int xs_gemm_batched(const void* x, int64_t ldx, int64_t sx, const void* w
     if (M == 0 || N == 0 || batch == 0) return 0;
     XS_REQUIRE(batch > 0 && batch <= 65535 && M > 0 && N > 0 && K > 0, "gemm_batched: %d x (%d x %d x %d)", batch, M, N, K);
     XS_REQUIRE(ldx >= K && ldw >= K && ldo >= N, "gemm_batched: a row stride is shorter than its row");
+    if (M <= 16 && dtype == XS_BF16 && K % 8 == 0 && ldx % 8 == 0 && sx % 8 == 0 && ldw % 8 == 0 && sw % 8 == 0 &&
+        ((uintptr_t)x | (uintptr_t)w) % 16 == 0) {
+        xs_launch(M <= 8 ? gemm_batched_few_rows_mma_kernel<1> : gemm_batched_few_rows_mma_kernel<2>, dim3(ceil_div_i(N, kFewRows), batch),
+                  dim3(kFewWarps * 32), 0, stream, (const __nv_bfloat16*)x, ldx, sx, (const __nv_bfloat16*)w, ldw, sw, (__nv_bfloat16*)out, ldo,
+                  so, M, N, K);
+        XS_LAUNCH_CHECK("gemm_batched (few rows)");
+        return 0;
+    }
     if (M <= 16 && (size_t)M * K * 4 <= 48 * 1024) {
         const int cols = 8;         // columns a block owns (8 warps, one each)
         XS_DISPATCH_DTYPE(dtype, TT,
@@ -879,7 +925,9 @@ __global__ void __launch_bounds__(256, 2) latent_attention_mma16_kernel(const La
     }
 }
 
-// One block per (token, head): the splits' maxima, sums and outputs into the final row.
+// One block per (token, head): the splits' maxima, sums and outputs into the final row. Two neighbouring columns a thread; the
+// first eight splits' values are asked for before the weights are known (128 rows of 512 columns on B200: 3.8 us; 10.7
+// with a column at a time behind the weights).
 __global__ void latent_attention_combine_kernel(const float* __restrict__ scratch, const float* __restrict__ sink,
                                                 const __nv_bfloat16* __restrict__ gate, int64_t ld_gate,
                                                 __nv_bfloat16* __restrict__ out, int64_t os_t, int64_t os_h, int H, int R,
@@ -890,6 +938,11 @@ __global__ void latent_attention_combine_kernel(const float* __restrict__ scratc
     __shared__ float norm_sm;
     const int tok = blockIdx.x / H, h = blockIdx.x % H;
     const float* src = scratch + (int64_t)blockIdx.x * splits * (R + 2);
+    float2 early[8];                  // (R is even, so a split's values start on 8-byte boundaries)
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+        early[s] = s < splits && 2 * (int)threadIdx.x < R ? *reinterpret_cast<const float2*>(src + (int64_t)s * (R + 2) + 2 + 2 * threadIdx.x)
+                                                          : make_float2(0.0f, 0.0f);
     if (threadIdx.x < 32) {           // splits <= 64: two per lane, all loads in flight at once
         const int s0 = threadIdx.x, s1 = threadIdx.x + 32;
         const float m0 = s0 < splits ? src[(int64_t)s0 * (R + 2)] : -INFINITY, m1 = s1 < splits ? src[(int64_t)s1 * (R + 2)] : -INFINITY;
@@ -909,11 +962,22 @@ __global__ void latent_attention_combine_kernel(const float* __restrict__ scratc
     __syncthreads();
     const float norm = norm_sm;
     __nv_bfloat16* dst = out + (int64_t)tok * os_t + (int64_t)h * os_h;
-    for (int c = threadIdx.x; c < R; c += blockDim.x) {
-        float v = 0.0f;
+    for (int c = 2 * threadIdx.x; c < R; c += 2 * blockDim.x) {
+        float2 v = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            if (s >= splits) break;
+            const float2 o = c < 2 * (int)blockDim.x ? early[s] : *reinterpret_cast<const float2*>(src + (int64_t)s * (R + 2) + 2 + c);
+            v.x = fmaf(o.x, weight[s], v.x);
+            v.y = fmaf(o.y, weight[s], v.y);
+        }
 #pragma unroll 8
-        for (int s = 0; s < splits; ++s) v = fmaf(src[(int64_t)s * (R + 2) + 2 + c], weight[s], v);
-        dst[c] = __float2bfloat16_rn(v * norm);
+        for (int s = 8; s < splits; ++s) {
+            const float2 o = *reinterpret_cast<const float2*>(src + (int64_t)s * (R + 2) + 2 + c);
+            v.x = fmaf(o.x, weight[s], v.x);
+            v.y = fmaf(o.y, weight[s], v.y);
+        }
+        *reinterpret_cast<__nv_bfloat162*>(dst + c) = __floats2bfloat162_rn(v.x * norm, v.y * norm);
     }
 }
 
@@ -984,7 +1048,7 @@ XS_API int xs_latent_attention_mma(const void* q_lat, int64_t qs_t, int64_t qs_h
 #undef XS_GO
     XS_LAUNCH_CHECK("latent_attention_mma");
     if (splits > 1) {
-        xs_launch(latent_attention_combine_kernel, dim3(T * H), dim3(128), 0, stream, (const float*)scratch, sink,
+        xs_launch(latent_attention_combine_kernel, dim3(T * H), dim3(R <= 256 ? 128 : 256), 0, stream, (const float*)scratch, sink,
                   (const __nv_bfloat16*)gate, ld_gate, (__nv_bfloat16*)out, os_t, os_h, H, R, splits);
         XS_LAUNCH_CHECK("latent_attention_combine");
     }

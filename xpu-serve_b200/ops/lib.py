@@ -94,7 +94,7 @@ def _signatures(lib) -> None:
         "xs_token_mix": [P, L, P, P, P, P, P, P, I, I, I, I, P],
         "xs_low_rank_decay": [P, L, P, I, P, P, I, I, I, I, I, F, P],
         "xs_decay_scan": [P, L, P, L, P, L, P, P, P, P, P, P, P, L, P, P, L, I, I, I, I, F, F, I, P, P, I, P, P, P],
-        "xs_mamba2_scan": [P, P, L, I, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
+        "xs_mamba2_scan": [P, P, L, I, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
         "xs_mamba2_scan_chunked": [P, P, L, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
     }
     for name, args in sig.items():
@@ -1323,9 +1323,9 @@ def mamba2_conv(proj: torch.Tensor, col0: int, taps_w: torch.Tensor, bias: Optio
 
 def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor,
                 d_skip: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, y: torch.Tensor,
-                heads: int, vdim: int, n_state: int, groups: int, chunks=None) -> None:
+                heads: int, vdim: int, n_state: int, groups: int, chunks=None, single: bool = False) -> None:
     """The recurrence over a step's tokens; y [T, heads * vdim] float32 takes y_t * silu(z_t). state: [*, heads,
-    n_state, vdim] float32. `chunks` = (chunk_seq [n, 3] int32, first_chunk [n_seqs + 1] int32, chunk_state, chunk_decay)
+    n_state, vdim] float32. `single`: every sequence brings exactly one token. `chunks` = (chunk_seq [n, 3] int32, first_chunk [n_seqs + 1] int32, chunk_state, chunk_decay)
     runs long pieces chunk by chunk side by side."""
     _need(xbc, "xbc", proj.dtype); _need(state, "state", torch.float32); _need(y, "y", torch.float32)
     for t, name in ((dt_bias, "dt_bias"), (a_log, "A_log"), (d_skip, "D")):
@@ -1340,8 +1340,8 @@ def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: tor
     if chunks is None:
         _check(load().xs_mamba2_scan(xbc.data_ptr(), proj.data_ptr(), proj.stride(0), int(dt_col), dt_bias.data_ptr(),
                                      a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), cu_seqlens.data_ptr(),
-                                     slots.data_ptr(), y.data_ptr(), n_seqs, heads, vdim, n_state, groups, _code(proj),
-                                     _stream()))
+                                     slots.data_ptr(), y.data_ptr(), n_seqs, heads, vdim, n_state, groups, int(single),
+                                     _code(proj), _stream()))
         return
     chunk_seq, first_chunk, chunk_state, chunk_decay = chunks
     _need(chunk_seq, "chunk_seq", torch.int32); _need(first_chunk, "first_chunk", torch.int32)

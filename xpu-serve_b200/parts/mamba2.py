@@ -97,7 +97,7 @@ class Mamba2Mixer(Mixer):
                       rt.ws.get("m2_chunk_state", (n, s.heads, s.state, s.vdim), torch.float32),
                       rt.ws.get("m2_chunk_decay", (n, s.heads), torch.float32))
         ops.mamba2_scan(xbc, proj, inner + C, self.dt_bias, self.a_log, self.d_skip, cache[1].storage, step.cu_seqlens,
-                        step.slots, y, s.heads, s.vdim, s.state, s.groups, chunks)
+                        step.slots, y, s.heads, s.vdim, s.state, s.groups, chunks, single=step.decode)
         yn = rt.ws.get("m2_normed", (T, inner), rt.act_dtype)
         ops.grouped_rmsnorm(y, self.w_norm, yn, s.norm_groups, s.eps)
         return rt.linear(yn, self.w_out, "mixer_out")
