@@ -250,7 +250,7 @@ class Runtime:
             else:
                 ops.gemm_generic(x, w, out, bias)
         elif out_dtype == torch.float32:
-            out.copy_(torch.mm(x, w.t(), out_dtype=torch.float32))
+            torch.mm(x, w.t(), out_dtype=torch.float32, out=out)
         else:
             torch.mm(x, w.t(), out=out)
         return out
