@@ -245,3 +245,22 @@ def test_mamba2_step(heads, P, N, G, seqs, dtype):
     assert gap(y, want) <= 4e-6 and gap(state[slots.long()], s) <= 2e-6
     rest = torch.tensor([i for i in range(seqs + 2) if i not in set(slots.tolist())], device=DEV)
     assert torch.equal(state[rest], state0[rest])
+
+
+@pytest.mark.parametrize("taps,C,col0,seqs", [(1, 16, 8, 2), (2, 24, 0, 1), (3, 1032, 16, 5), (4, 64, 8, 8), (5, 48, 8, 3), (4, 20, 4, 3)])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_mamba2_conv_of_single_tokens(taps, C, col0, seqs, dtype):
+    proj, w, bias = torch.randn(seqs, col0 + C + 8, device=DEV).to(dtype), torch.randn(C, taps, device=DEV), torch.randn(C, device=DEV)
+    state0 = torch.randn(seqs + 2, max(taps - 1, 1), C, device=DEV).to(dtype)
+    slots = torch.randperm(seqs + 2, device=DEV)[:seqs].to(torch.int32)
+    seq, cu = torch.arange(seqs, dtype=torch.int32, device=DEV), torch.arange(seqs + 1, dtype=torch.int32, device=DEV)
+    state, out = state0.clone(), torch.empty(seqs, C, device=DEV, dtype=dtype)
+    ops().mamba2_conv(proj, col0, w, bias, state, seq, cu, slots, out, single=True)
+    new = proj[:, None, col0:col0 + C]
+    rows = torch.cat([state0[slots.long()][:, :taps - 1], new], 1)
+    acc = (rows.double() * w.double().T[None]).sum(1) + bias.double()
+    assert gap(out, acc * torch.sigmoid(acc)) <= (2.0 ** -8 if dtype == BF else 2e-6)
+    want = state0.clone()
+    if taps > 1:
+        want[slots.long()] = rows[:, 1:]
+    assert torch.equal(state, want)

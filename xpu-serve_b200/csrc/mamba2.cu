@@ -59,41 +59,47 @@ __global__ void mamba2_conv_kernel(const T* __restrict__ proj, int64_t ld, int c
     out[(int64_t)t * C + c] = from_f32<T>(silu_f(acc));
 }
 
-// The same for bfloat16 with 8 channels a thread (16-byte loads and stores): C, col0 and ld multiples of 8.
-__global__ void mamba2_conv_bf16x8_kernel(const __nv_bfloat16* __restrict__ proj, int64_t ld, int col0,
-                                          const float* __restrict__ taps_w, const float* __restrict__ bias,
-                                          const __nv_bfloat16* __restrict__ state, const int32_t* __restrict__ seq_of_token,
-                                          const int32_t* __restrict__ cu_seqlens, const int32_t* __restrict__ slots,
-                                          __nv_bfloat16* __restrict__ out, int Tn, int C, int taps) {
+// The same for bfloat16 with 8 channels a thread (16-byte loads and stores): C, col0 and ld multiples of 8. SINGLE: every sequence
+// brings one token, and the kernel moves the sequence's state as well (it has the rows in registers). With the number of taps an
+// argument, the channels' taps were indexed in local memory: 8 tokens of 6,144 channels on B200 4.5 us; 7.4 before, and 5.1 for the
+// state's own kernel.
+template <int TAPS, bool SINGLE>
+__global__ void __launch_bounds__(128)
+mamba2_conv_bf16x8_kernel(const __nv_bfloat16* __restrict__ proj, int64_t ld, int col0, const float* __restrict__ taps_w,
+                          const float* __restrict__ bias, __nv_bfloat16* __restrict__ state, const int32_t* __restrict__ seq_of_token,
+                          const int32_t* __restrict__ cu_seqlens, const int32_t* __restrict__ slots, __nv_bfloat16* __restrict__ out, int C) {
     pdl_launch_dependents();
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
-    const int t = blockIdx.x;
     if (c >= C) return;
-    const int seq = seq_of_token[t];
-    const int local = t - cu_seqlens[seq];
-    const int64_t slot = slots[seq];
+    // (a decode step's token t of sequence t)
+    const int seq = SINGLE ? (int)blockIdx.x : seq_of_token[blockIdx.x];
+    const int t = SINGLE ? cu_seqlens[seq] : (int)blockIdx.x;
+    const int local = SINGLE ? 0 : t - cu_seqlens[seq];
+    __nv_bfloat16* st = state + (int64_t)slots[seq] * (TAPS - 1) * C + c;
     float acc[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = bias != nullptr ? bias[c + j] : 0.0f;
-    float wv[32];                                   // the 8 channels' taps, contiguous in memory (taps <= 4 here)
+    float wv[8 * TAPS];                             // the 8 channels' taps, contiguous in memory
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-        if (i < 2 * taps) *reinterpret_cast<float4*>(wv + 4 * i) = *reinterpret_cast<const float4*>(taps_w + (int64_t)c * taps + 4 * i);
+    for (int i = 0; i < 2 * TAPS; ++i) *reinterpret_cast<float4*>(wv + 4 * i) = *reinterpret_cast<const float4*>(taps_w + (int64_t)c * TAPS + 4 * i);
     pdl_wait();
+    uint4 raw[TAPS];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (k >= taps) break;
-        const int back = taps - 1 - k;
-        const __nv_bfloat16* src = local - back >= 0 ? proj + (int64_t)(t - back) * ld + col0 + c
-                                                      : state + (slot * (taps - 1) + (taps - 1 - (back - local))) * C + c;
-        const uint4 raw = *reinterpret_cast<const uint4*>(src);
-        const __nv_bfloat162* v2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    for (int k = 0; k < TAPS; ++k) {
+        const int back = TAPS - 1 - k;
+        const __nv_bfloat16* src = local - back >= 0 ? proj + (int64_t)(t - back) * ld + col0 + c : st + (int64_t)(TAPS - 1 - (back - local)) * C;
+        raw[k] = *reinterpret_cast<const uint4*>(src);
+    }
+#pragma unroll
+    for (int k = 0; k < TAPS; ++k) {
+        const __nv_bfloat162* v2 = reinterpret_cast<const __nv_bfloat162*>(&raw[k]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float2 f = __bfloat1622float2(v2[j]);
-            acc[2 * j] = fmaf(wv[(2 * j) * taps + k], f.x, acc[2 * j]);
-            acc[2 * j + 1] = fmaf(wv[(2 * j + 1) * taps + k], f.y, acc[2 * j + 1]);
+            acc[2 * j] = fmaf(wv[(2 * j) * TAPS + k], f.x, acc[2 * j]);
+            acc[2 * j + 1] = fmaf(wv[(2 * j + 1) * TAPS + k], f.y, acc[2 * j + 1]);
         }
+        if (SINGLE && k > 0) *reinterpret_cast<uint4*>(st + (int64_t)(k - 1) * C) = raw[k];
     }
     uint4 o;
     __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
@@ -331,7 +337,7 @@ __global__ void mamba2_scan_kernel(ScanArgs a) {
 // every `rows`-th row of the state (16-byte loads, eight of them in flight), so that the state streams through the whole CTA;
 // the rows' shares of y meet in shared memory and are added in the order of the threads' rows. Bound by the state's bytes, read
 // and written once; the kernel above keeps a column a thread (two warps a CTA at 64 columns, 4-byte loads, all rows in registers),
-// which is made for many tokens. Measured on B200 (8 sequences, 64 heads, a 128 x 64 state: 34 MB): 14.1 us, 22.6 there.
+// which is made for many tokens. Measured on B200 (8 sequences, 64 heads, a 128 x 64 state: 34 MB): 11.4 us, 22.6 there.
 template <typename T>
 __global__ void __launch_bounds__(256) mamba2_step_kernel(ScanArgs a) {
     __shared__ __align__(16) float part[256 * 4];
@@ -343,27 +349,34 @@ __global__ void __launch_bounds__(256) mamba2_step_kernel(ScanArgs a) {
     const T* proj = (const T*)a.proj + t * a.ld;
     float4* st = reinterpret_cast<float4*>(a.state + ((int64_t)a.slots[seq] * a.heads + h) * a.N * a.P) + c;
     const float bias = a.dt_bias[h], rate = -expf(a.a_log[h]), dskip = a.d_skip[h];
+    const T* B = xbc + inner + g * a.N;
+    const T* C = B + a.G * a.N;
     pdl_wait();
-    const float dt = softplus_f(to_f32(proj[a.dt_col + h]) + bias), da = expf(rate * dt);
     if (r < rows) {
-        float4 x, acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        x.x = dt * to_f32(xbc[h * a.P + 4 * c]);
-        x.y = dt * to_f32(xbc[h * a.P + 4 * c + 1]);
-        x.z = dt * to_f32(xbc[h * a.P + 4 * c + 2]);
-        x.w = dt * to_f32(xbc[h * a.P + 4 * c + 3]);
-        const T* B = xbc + inner + g * a.N;
-        const T* C = B + a.G * a.N;
+        // (the state's loads stand first: a warp issues in order, and would wait for the token's step size before them)
+        float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f), acc = x;
+        float da = 0.0f;
         for (int n0 = r; n0 < a.N; n0 += 8 * rows) {
             float4 S[8];
             float b[8], cc[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int n = n0 + u * rows;
+                if (n < a.N) S[u] = st[(int64_t)n * P4];
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int n = n0 + u * rows;
                 if (n < a.N) {
-                    S[u] = st[(int64_t)n * P4];
                     b[u] = to_f32(B[n]);
                     cc[u] = to_f32(C[n]);
                 }
+            }
+            if (n0 == r) {
+                const T raw[4] = {xbc[h * a.P + 4 * c], xbc[h * a.P + 4 * c + 1], xbc[h * a.P + 4 * c + 2], xbc[h * a.P + 4 * c + 3]};
+                const float dt = softplus_f(to_f32(proj[a.dt_col + h]) + bias);
+                da = expf(rate * dt);
+                x = make_float4(dt * to_f32(raw[0]), dt * to_f32(raw[1]), dt * to_f32(raw[2]), dt * to_f32(raw[3]));
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -436,15 +449,28 @@ int launch_scan(const ScanArgs& a, int units, cudaStream_t stream) {
 
 XS_API int xs_mamba2_conv(const void* proj, int64_t ld, int col0, const float* taps_w, const float* bias, void* state,
                           const int32_t* seq_of_token, const int32_t* cu_seqlens, const int32_t* slots, void* out, int T,
-                          int n_seqs, int C, int taps, int dtype, cudaStream_t stream) {
+                          int n_seqs, int C, int taps, int single, int dtype, cudaStream_t stream) {
     if (T == 0) return 0;
     XS_REQUIRE(C > 0 && taps >= 1 && taps <= kMaxTaps, "mamba2_conv: %d channels, %d taps (at most %d)", C, taps, kMaxTaps);
     XS_REQUIRE(n_seqs > 0 && C <= 65535 * 128, "mamba2_conv: %d tokens in %d sequences, %d channels", T, n_seqs, C);
     const int tiles = ceil_div_i(C, 128);
     if (dtype == XS_BF16 && taps <= 4 && (uintptr_t)taps_w % 16 == 0 && C % 8 == 0 && col0 % 8 == 0 && ld % 8 == 0 && (uintptr_t)proj % 16 == 0 && (uintptr_t)state % 16 == 0 &&
         (uintptr_t)out % 16 == 0) {
-        xs_launch(mamba2_conv_bf16x8_kernel, dim3(T, ceil_div_i(C / 8, 128)), dim3(128), 0, stream, (const __nv_bfloat16*)proj, ld,
-                  col0, taps_w, bias, (const __nv_bfloat16*)state, seq_of_token, cu_seqlens, slots, (__nv_bfloat16*)out, T, C, taps);
+        const bool moves = single && taps > 1 && T == n_seqs;
+#define XS_GO(TP, SG)                                                                                                                   \
+    xs_launch(mamba2_conv_bf16x8_kernel<TP, SG>, dim3(T, ceil_div_i(C / 8, 128)), dim3(128), 0, stream, (const __nv_bfloat16*)proj, ld, col0, \
+              taps_w, bias, (__nv_bfloat16*)state, seq_of_token, cu_seqlens, slots, (__nv_bfloat16*)out, C)
+        switch (taps) {
+            case 1: XS_GO(1, false); break;
+            case 2: if (moves) XS_GO(2, true); else XS_GO(2, false); break;
+            case 3: if (moves) XS_GO(3, true); else XS_GO(3, false); break;
+            default: if (moves) XS_GO(4, true); else XS_GO(4, false); break;
+        }
+#undef XS_GO
+        if (moves) {
+            XS_LAUNCH_CHECK("mamba2_conv");
+            return 0;
+        }
     } else {
         XS_DISPATCH_DTYPE(dtype, TT,
                           xs_launch(mamba2_conv_kernel<TT>, dim3(T, tiles), dim3(128), 0, stream, (const TT*)proj, ld, col0,

@@ -80,7 +80,7 @@ def _signatures(lib) -> None:
         "xs_latent_attention_generic": [P, L, L, P, P, P, I, P, P, P, L, P, P, L, L, I, I, I, I, I, F, I, I, P],
         "xs_gemm_batched": [P, L, L, P, L, L, P, L, L, I, I, I, I, I, P],
         "xs_latent_attention_mma": [P, L, L, P, P, P, I, P, P, P, L, P, P, L, L, P, L, I, I, I, I, I, I, I, F, I, I, P],
-        "xs_mamba2_conv": [P, L, I, P, P, P, P, P, P, P, I, I, I, I, I, P],
+        "xs_mamba2_conv": [P, L, I, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
         "xs_embed_pos": [P, P, I, P, P, P, I, I, F, P],
         "xs_causal_conv": [P, L, P, P, P, P, P, P, L, I, I, I, I, I, I, I, I, P],
         "xs_gated_add": [P, P, I, P, L, P, I, I, P],
@@ -1304,9 +1304,11 @@ def gemm_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
 
 # -------------------------------------------------------------------------------------- mamba-2
 def mamba2_conv(proj: torch.Tensor, col0: int, taps_w: torch.Tensor, bias: Optional[torch.Tensor], state: torch.Tensor,
-                seq_of_token: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, out: torch.Tensor) -> None:
+                seq_of_token: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, out: torch.Tensor,
+                single: bool = False) -> None:
     """out = silu(causal depthwise conv of proj[:, col0:col0 + C] + bias), inputs before the step from `state`
-    [*, taps - 1, C], which is then moved on. taps_w: [C, taps], the last column the current token's."""
+    [*, taps - 1, C], which is then moved on. taps_w: [C, taps], the last column the current token's. `single`: every sequence
+    brings exactly one token."""
     _need(out, "out", proj.dtype); _need(state, "state", proj.dtype); _need(taps_w, "taps", torch.float32)
     T, C = out.shape
     taps = taps_w.shape[1]
@@ -1318,7 +1320,7 @@ def mamba2_conv(proj: torch.Tensor, col0: int, taps_w: torch.Tensor, bias: Optio
         _need(bias, "bias", torch.float32)
     _check(load().xs_mamba2_conv(proj.data_ptr(), proj.stride(0), int(col0), taps_w.data_ptr(), _ptr(bias), state.data_ptr(),
                                  seq_of_token.data_ptr(), cu_seqlens.data_ptr(), slots.data_ptr(), out.data_ptr(), T,
-                                 slots.numel(), C, taps, _code(proj), _stream()), kernels=2 if taps > 1 else 1)
+                                 slots.numel(), C, taps, int(single), _code(proj), _stream()), kernels=1 if taps == 1 or single else 2)
 
 
 def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor,

@@ -87,7 +87,7 @@ class Mamba2Mixer(Mixer):
         proj = rt.linear(x, self.w_in, "m2_proj")
         xbc = rt.ws.get("m2_xbc", (T, C), rt.act_dtype)
         ops.mamba2_conv(proj, inner, self.taps, self.conv_bias, cache[0].storage, step.seq_of_token, step.cu_seqlens,
-                        step.slots, xbc)
+                        step.slots, xbc, single=step.decode)
         y = rt.ws.get("m2_y", (T, inner), torch.float32)
         chunks = None
         if self.chunk > 0 and not step.fixed_shape and not step.decode and step.max_q_len >= 2 * self.chunk:
