@@ -153,12 +153,25 @@ class Model:
                      dtype=self.rt.act_dtype, device=self.rt.device)
 
     # ------------------------------------------------------------------ step
-    def check_tokens(self, token_lists: Sequence[Sequence[int]]) -> None:
+    def check_tokens(self, token_lists: Sequence[Sequence[int]]) -> List[Sequence[int]]:
+        """The lists again, long ones as arrays of 64-bit ids (a look at each token in turn costs a prompt of 2,048 tokens a
+        quarter of a millisecond in which the device waits, and the step's description wants the array anyway)."""
         V = self.spec.vocab
+        out: List[Sequence[int]] = []
         for toks in token_lists:
+            if len(toks) >= 32:
+                try:
+                    ids = np.asarray(toks, dtype=np.int64)
+                except (TypeError, ValueError, OverflowError):
+                    ids = None
+                if ids is not None and ids.ndim == 1 and int(ids.min()) >= 0 and int(ids.max()) < V:
+                    out.append(ids)
+                    continue
             for t in toks:
                 if not 0 <= int(t) < V:
                     raise ValueError(f"token id {int(t)} outside the vocabulary ({V})")
+            out.append(toks)
+        return out
 
     def step(self, cache: Cache, slots: Sequence[int], token_lists: Sequence[Sequence[int]],
              want: Optional[Sequence[Sequence[int]]] = None) -> torch.Tensor:
@@ -172,8 +185,12 @@ class Model:
             want = [[len(t) - 1] for t in token_lists]
         if len(slots) != len(token_lists) or len(want) != len(slots):
             raise ValueError("a step needs one token list and one list of wanted places per slot")
-        self.check_tokens(token_lists)
+        token_lists = self.check_tokens(token_lists)
         for toks, places in zip(token_lists, want):
+            if len(places) >= 32:
+                at = np.asarray(places)
+                if at.ndim == 1 and at.dtype.kind == "i" and int(at.min()) >= 0 and int(at.max()) < len(toks):
+                    continue
             for p in places:
                 if not 0 <= int(p) < len(toks):
                     raise ValueError(f"wanted place {p} is not among the {len(toks)} tokens of the step")

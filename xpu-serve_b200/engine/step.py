@@ -75,7 +75,8 @@ class StepStager:
         T = int(q_lens.sum())
         cu = np.zeros(n + 1, dtype=np.int64)
         np.cumsum(q_lens, out=cu[1:])
-        want_rows = np.asarray([int(cu[i]) + int(p) for i, places in enumerate(want) for p in places], dtype=np.int64)
+        rows = [cu[i] + np.asarray(places, dtype=np.int64) for i, places in enumerate(want) if len(places)]
+        want_rows = np.concatenate(rows) if rows else np.zeros(0, dtype=np.int64)
         tables = {gi: cache.page_table(gi, slots) for gi in cache.kv_groups}
         flat = np.concatenate([np.asarray(t, dtype=np.int64) for t in token_lists]) if T else np.zeros(0, np.int64)
         seq_of = np.repeat(np.arange(n, dtype=np.int64), q_lens)
