@@ -183,6 +183,21 @@ def test_experts_of_few_tokens(T, top, E, F, H, act):
     assert gap(y, (rows * wts.double()[:, None]).view(T, top, H).sum(1)) <= 2.0 ** -8
 
 
+@pytest.mark.parametrize("M,F,K", [(1, 8, 8), (3, 24, 264), (8, 1024, 2048), (8, 16, 8192), (9, 40, 1032), (16, 1024, 2048)])
+@pytest.mark.parametrize("slices", [1, 4])
+def test_clamped_unit_of_few_rows(M, F, K, slices):
+    slices = slices if K > 1024 else 1
+    x, w = torch.randn(M, K, device=DEV).to(BF), (torch.randn(2 * F, K, device=DEV) * (2.0 / K) ** 0.5).to(BF)
+    scratch = torch.zeros(ops().gemm_small_m_scratch_bytes(M, 2 * F, slices), device=DEV, dtype=torch.uint8)
+    out = torch.full((M, F + 8), 7.0, device=DEV, dtype=BF)
+    for _ in range(2):
+        ops().gemm_small_m_clamped(x, w, out[:, :F], 1.5, 1.702, 1.0, ksplit=slices, scratch=scratch if slices > 1 else None)
+    g, u = (x.double() @ w.double().T).view(M, F // 8, 2, 8).unbind(2)
+    g, u = g.reshape(M, F).clamp(max=1.5), u.reshape(M, F).clamp(-1.5, 1.5)
+    assert gap(out[:, :F], g * torch.sigmoid(1.702 * g) * (u + 1.0)) <= 2.0 ** -8
+    assert bool((out[:, F:] == 7.0).all())
+
+
 def test_experts_rows_do_not_depend_on_the_step():
     E, F, H, top = 6, 64, 256, 2
     x = torch.randn(8, H, device=DEV).to(BF)

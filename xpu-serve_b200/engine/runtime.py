@@ -164,12 +164,12 @@ class Runtime:
         return ops.gemm_tc_supports(x.shape[0], w.shape[0], x.shape[1], x.stride(0), w.stride(0))
 
     def few_rows_product(self, x, w, out, bias=None, swiglu: bool = False, residual=None, next_w=None, next_x=None,
-                         out_ssq=None, conv=None, argmax_into=None) -> None:
+                         out_ssq=None, conv=None, argmax_into=None, clamp=None) -> None:
         """The library's weight-streaming product, with K cut over several CTAs where the output is
         narrow; the partial sums meet in one zero-initialised scratch buffer that lives as long as
         the runtime (its tail holds the kernel's counters). `x` may be a Prenormed input; `residual`
         (the float32 stream) takes the result instead of `out`, with `next_*` / `out_ssq` as in
-        ops.gemm_small_m."""
+        ops.gemm_small_m. `clamp` (limit, alpha, shift): the clamped unit behind a gate and up product."""
         norm = {}
         if hasattr(x, "ssq"):
             norm = dict(in_ssq=x.ssq, in_width=x.width, in_eps=x.eps)
@@ -177,6 +177,9 @@ class Runtime:
         ksplit = ops.gemm_small_m_ksplit(x.shape[0], w.shape[0], x.shape[1], self.sm_count)
         if ksplit > 1 and ops.gemm_small_m_scratch_bytes(x.shape[0], w.shape[0], ksplit) > self.gemm_scratch.numel():
             ksplit = 1
+        if clamp is not None:
+            ops.gemm_small_m_clamped(x, w, out, *clamp, ksplit=ksplit, scratch=self.gemm_scratch if ksplit > 1 else None)
+            return
         if conv is not None:
             ksplit = 1          # the convolution behind the product counts whole tiles
             conv = dict(conv, counters=self.conv_counters)

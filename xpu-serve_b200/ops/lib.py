@@ -50,6 +50,7 @@ def _signatures(lib) -> None:
         "xs_attention_mma": [P, P, P, I, P, P, P, L, P, P, L, I, I, I, I, I, I, I, F, I, I, P],
         "xs_attention_tc": [P, P, L, P, I, P, P, P, L, P, L, I, I, I, I, I, I, I, I, F, F, I, I, I, I, I, P, P],
         "xs_gemm_small_m": [P, P, P, P, P, I, I, I, I, L, L, L, I, I, P, L, P],
+        "xs_gemm_small_m_clamped": [P, P, P, I, I, I, L, L, L, I, P, L, F, F, F, P],
         "xs_gemm_small_m_normed": [P, P, P, P, P, I, I, I, I, L, L, L, I, I, P, L, P, I, I, F, P, P, L, P, P],
         "xs_gemm_small_m_ex": [P, P, P, P, P, I, I, I, I, L, L, L, I, I, P, L, P, I, I, F, P, P, L, P,
                                P, P, P, P, P, P, I, I, P, P, P, P],
@@ -654,6 +655,21 @@ def gemm_small_m(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], 
         x.stride(0), w.stride(0), target.stride(0), 2 if swiglu == "relu_squared" else 3 if swiglu == "gelu_tanh" else 1 if swiglu else 0, int(ksplit), _ptr(scratch),
         0 if scratch is None else scratch.numel() * scratch.element_size(), _ptr(in_ssq), in_tiles, int(in_width),
         float(in_eps), _ptr(next_w), _ptr(next_x), ld_next, _ptr(out_ssq), *cv, *am, _stream()))
+
+
+def gemm_small_m_clamped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, limit: float, alpha: float, shift: float,
+                         ksplit: int = 1, scratch: Optional[torch.Tensor] = None) -> None:
+    """out[M, N / 2] = the clamped unit (`clamped_glu`) of x . w^T for M <= 16, bfloat16, w stacked as blocks of 8 gate and 8 up
+    rows. `ksplit` and `scratch` as in gemm_small_m."""
+    for t, name in ((x, "x"), (w, "w"), (out, "out")):
+        if not t.is_cuda or t.dim() != 2 or t.stride(1) != 1 or t.dtype != torch.bfloat16:
+            raise KernelError(f"gemm (few rows): {name} must be a bfloat16 CUDA matrix with contiguous rows")
+    M, K = x.shape
+    if w.shape[1] != K or tuple(out.shape) != (M, w.shape[0] // 2):
+        raise KernelError(f"gemm (few rows): x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    _check(load().xs_gemm_small_m_clamped(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, w.shape[0], K, x.stride(0), w.stride(0), out.stride(0),
+                                          int(ksplit), _ptr(scratch), 0 if scratch is None else scratch.numel() * scratch.element_size(),
+                                          float(limit), float(alpha), float(shift), _stream()))
 
 
 def gemm_small_m_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor],

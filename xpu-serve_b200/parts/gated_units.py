@@ -62,6 +62,8 @@ class ClampedGLU(FeedForward):
         act = rt.ws.get("ffn_act", (y.shape[0], s.intermediate), rt.act_dtype)
         if self.interleave and rt.tensor_core_product(y, self.w_gate_up, fused=True):
             ops.gemm_tc_clamped(y, self.w_gate_up, act, s.limit, s.alpha, s.up_shift)
+        elif self.interleave and rt.few_rows(y, self.w_gate_up):
+            rt.few_rows_product(y, self.w_gate_up, act, clamp=(s.limit, s.alpha, s.up_shift))
         else:
             gu = rt.linear(y, self.w_gate_up, "ffn_gate_up")
             ops.clamped_glu(gu, act, s.limit, s.alpha, s.up_shift, self.interleave)
