@@ -55,22 +55,29 @@ struct GemmTcParams {
 };
 
 // 1 / v to one unit in the last place, by the hardware's reciprocal (the division's own steps for odd ranges and the last half
-// unit cost the gated epilogue a third of its instructions, for a result that is rounded to bfloat16).
+// unit cost the gated epilogue a third of its instructions, for a result that is rounded to bfloat16: against 64 bits the bfloat16
+// outputs' errors are the same in every digit, float32 outputs' would be 10 to 17 % larger, so those keep the division).
 __device__ __forceinline__ float near_rcp(float v) {
     float r;
     asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
 
+template <bool DIVIDE>
 __device__ __forceinline__ float gated_unit(const GemmTcParams& p, float g, float u) {
     // (0.5 (1 + tanh(a)) = 1 / (1 + exp(-2 a)): the tanh form of gelu costs one exponential, as silu does)
     if (p.glu_act == 1) return __fdividef(g * u, 1.0f + __expf(-1.5957691216057308f * g * fmaf(0.044715f * g, g, 1.0f)));
     if (p.glu_limit > 0.0f) {
         g = fminf(g, p.glu_limit);
         u = fminf(fmaxf(u, -p.glu_limit), p.glu_limit);
-        return g * near_rcp(1.0f + __expf(-p.glu_alpha * g)) * (u + p.glu_shift);
+        const float d = 1.0f + __expf(-p.glu_alpha * g);
+        return (DIVIDE ? g / d : g * near_rcp(d)) * (u + p.glu_shift);
     }
-    return g * near_rcp(1.0f + __expf(-g)) * u;
+    const float d = 1.0f + __expf(-g);
+    return (DIVIDE ? g / d : g * near_rcp(d)) * u;
+}
+__device__ __forceinline__ float gated_unit_of(const GemmTcParams& p, float g, float u) {
+    return p.out_f32 ? gated_unit<true>(p, g, u) : gated_unit<false>(p, g, u);
 }
 
 // Instruction descriptor of this file's single-CTA products: M = 128, N = n.
@@ -90,7 +97,7 @@ __device__ __forceinline__ void emit(const GemmTcParams& p, float v, int row, in
     if (p.epilogue == EPI_SWIGLU) {
         const float up = __shfl_xor_sync(0xffffffffu, v, 8);
         if ((lane & 8) == 0 && row + 8 < p.N && token < p.T) {
-            const float a = gated_unit(p, v, up);
+            const float a = gated_unit_of(p, v, up);
             const int64_t at = (int64_t)token * p.ldo + (row >> 4) * 8 + (row & 7);
             if (p.out_f32) ((float*)p.out)[at] = a; else ((__nv_bfloat16*)p.out)[at] = __float2bfloat16_rn(a);
         }
@@ -131,7 +138,7 @@ __device__ __forceinline__ void emit16(const GemmTcParams& p, const uint32_t* r,
     if (p.epilogue == EPI_SWIGLU) {   // rows f0..f0+7 are gates, f0+8..f0+15 their up rows; N is a multiple of 16
         float a[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = gated_unit(p, v[j], v[j + 8]);
+        for (int j = 0; j < 8; ++j) a[j] = gated_unit_of(p, v[j], v[j + 8]);
         const int64_t at = (int64_t)token * p.ldo + (f0 >> 1);
         if (p.out_f32) {
             float* o = (float*)p.out + at;
@@ -187,7 +194,8 @@ __device__ __forceinline__ void emit16(const GemmTcParams& p, const uint32_t* r,
 
 // Thirty-two of them (f0 a multiple of 32), in whole 32-byte sectors where the rows allow it.
 __device__ __forceinline__ void emit32(const GemmTcParams& p, const uint32_t* r, int token, int f0) {
-    if (p.vec < 2 || p.bias != nullptr || f0 + 32 > p.N || token >= p.T || (p.epilogue != EPI_SWIGLU && p.epilogue != EPI_STORE)) {
+    if (p.vec < 2 || p.bias != nullptr || f0 + 32 > p.N || token >= p.T ||
+        (p.epilogue != EPI_STORE && (p.epilogue != EPI_SWIGLU || p.out_f32))) {
         emit16(p, r, token, f0);
         emit16(p, r + 16, token, f0 + 16);
         return;
@@ -197,20 +205,13 @@ __device__ __forceinline__ void emit32(const GemmTcParams& p, const uint32_t* r,
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
             const int g = (j & 7) + (j >> 3) * 16;
-            a[j] = gated_unit(p, __uint_as_float(r[g]), __uint_as_float(r[g + 8]));
+            a[j] = gated_unit<false>(p, __uint_as_float(r[g]), __uint_as_float(r[g + 8]));
         }
         const int64_t at = (int64_t)token * p.ldo + (f0 >> 1);
-        uint32_t o[16];
-        if (p.out_f32) {
+        uint32_t o[8];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(a[j]);
-            store_32((float*)p.out + at, o);
-            store_32((float*)p.out + at + 8, o + 8);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = pack_bf16(a[2 * j], a[2 * j + 1]);
-            store_32((__nv_bfloat16*)p.out + at, o);
-        }
+        for (int j = 0; j < 8; ++j) o[j] = pack_bf16(a[2 * j], a[2 * j + 1]);
+        store_32((__nv_bfloat16*)p.out + at, o);
         return;
     }
     const int64_t at = (int64_t)token * p.ldo + f0;
