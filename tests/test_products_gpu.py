@@ -125,21 +125,46 @@ def test_many_token_product_stores(T, N, pad, form):
     assert bool((out[:, cols:] == 7.0).all())
 
 
-def test_gated_epilogue_far_gates():
-    """Gates where the exponential is zero, huge or infinite."""
-    gates = torch.tensor([0.0, -80.0, -88.0, -88.6, -100.0, -3e4, 80.0, 100.0, 3e4], device=DEV)
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+@pytest.mark.parametrize("N,pad", [(16, 0), (64, 0), (96, 8), (272, 3)])
+@pytest.mark.parametrize("act", ["silu", "clamped"])
+def test_gated_epilogue_far_gates(dtype, N, pad, act):
+    """Gates where the exponential is zero, huge or infinite, on the 32-column stores (rows on 32 bytes) and off them."""
+    gates = torch.tensor([0.0, -1.0, -50.0, -80.0, -88.0, -88.6, -100.0, -3e4, 80.0, 100.0, 3e4], device=DEV)
     T, K = 130, 16
     x = torch.zeros(T, K, device=DEV, dtype=BF)
     x[:, 0] = gates[torch.arange(T, device=DEV) % len(gates)].to(BF)
     x[:, 1] = 3.0
-    w = torch.zeros(16, K, device=DEV, dtype=BF)
-    w[:8, 0], w[8:, 1] = 1.0, 1.0
-    out = torch.empty(T, 8, device=DEV)
-    ops().gemm_tc(x, w, out, epilogue=ops().EPI_SWIGLU)
+    w = torch.zeros(N // 16, 2, 8, K, device=DEV, dtype=BF)
+    w[:, 0, :, 0], w[:, 1, :, 1] = 1.0, 1.0
+    w = w.view(N, K)
+    out = torch.empty(T, N // 2 + pad, device=DEV, dtype=dtype)[:, :N // 2]
     g = x[:, :1].double()
-    assert gap(out, (g * torch.sigmoid(g) * 3.0).expand(T, 8)) <= 2.0 ** -20
-    small = g[:, 0] < -10
-    assert ((out[small].double() - (g * torch.sigmoid(g) * 3.0)[small]).abs() <= 1e-30).all()
+    if act == "clamped":
+        ops().gemm_tc_clamped(x, w, out, 7.0, 1.702, 1.0)
+        want = g.clamp(max=7.0) * torch.sigmoid(1.702 * g.clamp(max=7.0)) * 4.0
+    else:
+        ops().gemm_tc(x, w, out, epilogue=ops().EPI_SWIGLU)
+        want = g * torch.sigmoid(g) * 3.0
+    assert torch.isfinite(out).all()
+    # (the exponential's argument is some tens, rounded to 2^-24 of itself; far out only its size counts)
+    limit = want.abs() * (2.0 ** -8 if dtype == BF else 2.0 ** -17) + 1e-30
+    assert ((out.double() - want).abs() <= limit).all()
+
+
+@pytest.mark.parametrize("T", [7, 130, 400])      # (the epilogues of few tokens, of many and of pairs of CTAs)
+@pytest.mark.parametrize("act", ["silu", "clamped"])
+def test_gated_epilogue_rounds_once(T, act):
+    """bfloat16 outputs are the float32 outputs rounded: the gated unit is no less exact where its result is rounded."""
+    N, K = 1024, 256
+    x, w = torch.randn(T, K, device=DEV).to(BF), (torch.randn(N, K, device=DEV) * 0.125).to(BF)
+    exact, rounded = torch.empty(T, N // 2, device=DEV), torch.empty(T, N // 2, device=DEV, dtype=BF)
+    for out in (exact, rounded):
+        if act == "clamped":
+            ops().gemm_tc_clamped(x, w, out, 7.0, 1.702, 1.0)
+        else:
+            ops().gemm_tc(x, w, out, epilogue=ops().EPI_SWIGLU)
+    assert torch.equal(rounded, exact.to(BF))
 
 
 # ------------------------------------------------------------------------------------------- few tokens' experts

@@ -54,30 +54,17 @@ struct GemmTcParams {
     int glu_act;              // 1: the gate passes the tanh form of gelu instead (no limit)
 };
 
-// 1 / v to one unit in the last place, by the hardware's reciprocal (the division's own steps for odd ranges and the last half
-// unit cost the gated epilogue a third of its instructions, for a result that is rounded to bfloat16: against 64 bits the bfloat16
-// outputs' errors are the same in every digit, float32 outputs' would be 10 to 17 % larger, so those keep the division).
-__device__ __forceinline__ float near_rcp(float v) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
-    return r;
-}
-
-template <bool DIVIDE>
+// (divisions: by the hardware's reciprocal alone the result before its rounding to bfloat16 was up to 17 % further from 64 bits,
+// 5.6e-8 of its rms against 4.8e-8)
 __device__ __forceinline__ float gated_unit(const GemmTcParams& p, float g, float u) {
     // (0.5 (1 + tanh(a)) = 1 / (1 + exp(-2 a)): the tanh form of gelu costs one exponential, as silu does)
     if (p.glu_act == 1) return __fdividef(g * u, 1.0f + __expf(-1.5957691216057308f * g * fmaf(0.044715f * g, g, 1.0f)));
     if (p.glu_limit > 0.0f) {
         g = fminf(g, p.glu_limit);
         u = fminf(fmaxf(u, -p.glu_limit), p.glu_limit);
-        const float d = 1.0f + __expf(-p.glu_alpha * g);
-        return (DIVIDE ? g / d : g * near_rcp(d)) * (u + p.glu_shift);
+        return g / (1.0f + __expf(-p.glu_alpha * g)) * (u + p.glu_shift);
     }
-    const float d = 1.0f + __expf(-g);
-    return (DIVIDE ? g / d : g * near_rcp(d)) * u;
-}
-__device__ __forceinline__ float gated_unit_of(const GemmTcParams& p, float g, float u) {
-    return p.out_f32 ? gated_unit<true>(p, g, u) : gated_unit<false>(p, g, u);
+    return g / (1.0f + __expf(-g)) * u;
 }
 
 // Instruction descriptor of this file's single-CTA products: M = 128, N = n.
@@ -97,7 +84,7 @@ __device__ __forceinline__ void emit(const GemmTcParams& p, float v, int row, in
     if (p.epilogue == EPI_SWIGLU) {
         const float up = __shfl_xor_sync(0xffffffffu, v, 8);
         if ((lane & 8) == 0 && row + 8 < p.N && token < p.T) {
-            const float a = gated_unit_of(p, v, up);
+            const float a = gated_unit(p, v, up);
             const int64_t at = (int64_t)token * p.ldo + (row >> 4) * 8 + (row & 7);
             if (p.out_f32) ((float*)p.out)[at] = a; else ((__nv_bfloat16*)p.out)[at] = __float2bfloat16_rn(a);
         }
@@ -138,7 +125,7 @@ __device__ __forceinline__ void emit16(const GemmTcParams& p, const uint32_t* r,
     if (p.epilogue == EPI_SWIGLU) {   // rows f0..f0+7 are gates, f0+8..f0+15 their up rows; N is a multiple of 16
         float a[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = gated_unit_of(p, v[j], v[j + 8]);
+        for (int j = 0; j < 8; ++j) a[j] = gated_unit(p, v[j], v[j + 8]);
         const int64_t at = (int64_t)token * p.ldo + (f0 >> 1);
         if (p.out_f32) {
             float* o = (float*)p.out + at;
@@ -205,7 +192,7 @@ __device__ __forceinline__ void emit32(const GemmTcParams& p, const uint32_t* r,
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
             const int g = (j & 7) + (j >> 3) * 16;
-            a[j] = gated_unit<false>(p, __uint_as_float(r[g]), __uint_as_float(r[g + 8]));
+            a[j] = gated_unit(p, __uint_as_float(r[g]), __uint_as_float(r[g + 8]));
         }
         const int64_t at = (int64_t)token * p.ldo + (f0 >> 1);
         uint32_t o[8];
@@ -230,9 +217,10 @@ __device__ __forceinline__ void emit32(const GemmTcParams& p, const uint32_t* r,
 // One epilogue warp's share of a tile of the many-token kernels: its 32 lanes of tensor memory (tokens), half of the tile's BN
 // columns, 32 at a time; the next 32 are on their way while these leave. `handed_back` is called when the last of them are in
 // registers. What the gated epilogue costs decides whether the next tile's products hide it: a 256 x 256 tile of K = 1024 is
-// 4.4 us of tensor-core time, and with four warps, a division an output and 16-byte stores the epilogue took 15 us. Measured on
-// B200 with the gated epilogue (us, before -> now): 8,192 tokens N 13312 K 1024 352 -> 196 (1.14 PFLOP/s; 167 storing the product
-// as it is, the vendor's product 165), 8,192 x 16384 x 2048 452 -> 390, 2,048 x 16384 x 2048 124 -> 104.
+// 4.4 us of tensor-core time, and with four warps and 16-byte stores the epilogue took 15 us. Measured on B200 with the gated
+// epilogue (us, four warps -> now, L2 flushed): 8,192 tokens N 13312 K 1024 366 -> 257 (0.87 PFLOP/s; 159 storing the product as
+// it is, the vendor's product 159), 8,192 x 16384 x 2048 452 -> 383, 2,048 x 16384 x 2048 130 -> 112. (The divisions are what is
+// left of it: multiplied by an approximate reciprocal the first took 222.)
 template <int BN, typename F>
 __device__ __forceinline__ void drain_half(const GemmTcParams& p, uint32_t acc, int half, int token, bool live, int f0, F handed_back) {
     constexpr int kParts = BN / 64;
