@@ -96,6 +96,32 @@ def test_float32_attention(H, G, D, DV, planes, window, keep, plus, cap, lens):
     assert gap(out, ref) <= 4e-6      # (scores of a few units: 2^-24 of them through the exponential, on top of the sums)
 
 
+@pytest.mark.parametrize("H,G,D,DV,window,keep,plus", [(8, 4, 64, 64, 0, 0, 0), (8, 2, 32, 20, 300, 70, 1), (6, 2, 128, 64, 0, 0, 0),
+                                                       (4, 2, 256, 256, 0, 0, 0)])
+@pytest.mark.parametrize("keys", [1, 33, 130, 520, 700])
+def test_float32_attention_does_not_depend_on_the_step(H, G, D, DV, window, keep, plus, keys):
+    """A token alone and among more (token, head) pairs than a launch gives a warp a group: the same bits."""
+    page, P, T = 64, 11, 200
+    pool = torch.randn(2 * P, G * page * (D + DV), device=DEV)
+    pages = torch.randperm(2 * P, device=DEV).to(torch.int32).view(2, P)
+    q = torch.randn(T, H, D, device=DEV)
+    seq = (torch.arange(T, device=DEV) % 2).to(torch.int32)
+    pos = torch.randint(0, 700, (T,), device=DEV).to(torch.int32)
+    pos[77] = keys - 1
+    assert T * H > 4 * 148 >= H
+
+    def attend(t0, n):
+        out = torch.empty(n, H, DV, device=DEV)
+        qs, ss, ps = q[t0:t0 + n].contiguous(), seq[t0:t0 + n].clone(), pos[t0:t0 + n].clone()
+        ops()._check(ops().load().xs_attention_generic(
+            qs.data_ptr(), pool.data_ptr(), pages.data_ptr(), P, ss.data_ptr(), ps.data_ptr(), None, 0, out.data_ptr(), H * DV, n, H, G, D,
+            DV, 2, page, D ** -0.5, 0.0, window, keep, plus, 0, 0, ops()._stream()))
+        torch.cuda.synchronize()
+        return out
+
+    assert torch.equal(attend(77, 1)[0], attend(0, T)[77])
+
+
 # --------------------------------------------------------------------------- tcgen05 product, many tokens: the store paths
 @pytest.mark.parametrize("T,N", [(65, 48), (128, 272), (129, 256), (300, 528), (1000, 80)])
 @pytest.mark.parametrize("pad", [0, 8, 1])

@@ -319,13 +319,19 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, const T* __res
     }
 }
 
-// The same in float32 for head sizes that are multiples of 4 up to 32 * PIECES: a CTA per (token, q head), whose warps take
-// the token's key blocks of 32 in turn and merge their maxima, sums and outputs in shared memory. Eight lanes share a key: each
+// The same in float32 for head sizes that are multiples of 4 up to 32 * PIECES: a CTA per (token, q head). The token's key blocks
+// of 32 are dealt to kAttnF32Groups groups in turn; the groups' maxima, sums and outputs meet in shared memory in the groups' order.
+// The CTA's warps share the groups, so how many warps a launch has (a decode step's few pairs want one a group, a prompt's many
+// want four in all) changes no bit of a token's result. Eight lanes share a key: each
 // holds four neighbouring channels of every 32, so a warp reads 128 contiguous bytes of four keys at a time, a score is three
 // shuffles, and the weighted sum needs none until the end. The kernel above is bound by a serial chain (one warp walks all of a
 // token's keys, a lane reads a whole key row by itself, 4 bytes at a time).
-// Measured on B200 (350M shape: 16 heads over 8, head size 64; four sequences of up to 512 keys, one prompt step and 16 decode
-// steps): 456 -> 28 us a launch on average.
+// Measured on B200 (350M shape: 16 heads over 8, head size 64): four sequences of up to 512 keys, one prompt step and 16 decode
+// steps: 456 -> 27 us a launch on average; four tokens of 512 keys 14.4 us, 1,126 prompt tokens of up to 512 keys 234 us (227 with
+// one group a warp, whose bits would then depend on the launch), a prompt of 2,048 1.44 ms (1.41).
+template <int PIECES>
+constexpr int kAttnF32Groups = PIECES <= 2 ? 16 : 8;
+
 template <int PIECES>
 __global__ void attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ pool,
                                      const int32_t* __restrict__ page_table, int P, const int32_t* __restrict__ seq_of_token,
@@ -333,7 +339,8 @@ __global__ void attention_f32_kernel(const float* __restrict__ q, const float* _
                                      float* __restrict__ out, int64_t ld_out, int Hq, int Hkv, int D, int DV, int planes,
                                      int page_size, float scale, float softcap, int window, int keep, int plus_one,
                                      int gate_channels) {
-    extern __shared__ __align__(16) float merge_sm[];     // [warps][DV] outputs, then [warps] maxima, [warps] sums
+    constexpr int G = kAttnF32Groups<PIECES>;
+    extern __shared__ __align__(16) float merge_sm[];     // [G][DV] outputs, then [G] maxima, [G] sums, [G] weights
     pdl_launch_dependents();
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane & 7, kq = lane >> 3;
@@ -345,120 +352,135 @@ __global__ void attention_f32_kernel(const float* __restrict__ q, const float* _
     const int64_t k_at = (int64_t)kvh * page_size * D;
     const int64_t v_at = planes == 1 ? k_at : (int64_t)Hkv * page_size * D + (int64_t)kvh * page_size * DV;
     pdl_wait();                                            // (the step's description is written before the step's first kernel)
-    float4 qv[PIECES], acc[PIECES];
+    float4 qv[PIECES];
 #pragma unroll
     for (int u = 0; u < PIECES; ++u) {
         const int d = sub * 4 + 32 * u;
         qv[u] = d < D ? *reinterpret_cast<const float4*>(q + ((int64_t)t * Hq + h) * D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
         qv[u].x *= scale; qv[u].y *= scale; qv[u].z *= scale; qv[u].w *= scale;
-        acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     const int lo = xs_first_visible(pos, window);
     const int kept = min(keep, lo);
     const int kept_blocks = (kept + 31) >> 5, blocks = kept_blocks + ((pos + 1 - lo + 31) >> 5);
-    float m = -INFINITY, l = 0.0f;
-    for (int b = warp; b < blocks; b += warps) {
-        const bool early = b < kept_blocks;
-        const int j0 = early ? b * 32 : lo + (b - kept_blocks) * 32;
-        const int end = early ? kept : pos + 1;
-        const float* row[8];
-        float s[8];
+    const int used = min(G, blocks);                       // groups that have a block
+    float* maxima = merge_sm + G * DV;
+    float* sums = maxima + G;
+    float* weights = sums + G;
+    for (int group = warp; group < used; group += warps) {
+        float4 acc[PIECES];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int j = min(j0 + i * 4 + kq, end - 1);   // (a place past the end reads the last key and counts nothing)
-            const int page = j / page_size;
-            row[i] = pool + table[page] * page_elems + (int64_t)(j - page * page_size) * D + k_at;
-        }
+        for (int u = 0; u < PIECES; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        float m = -INFINITY, l = 0.0f;
+        for (int b = group; b < blocks; b += G) {
+            const bool early = b < kept_blocks;
+            const int j0 = early ? b * 32 : lo + (b - kept_blocks) * 32;
+            const int end = early ? kept : pos + 1;
+            const float* row[8];
+            float s[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            float dot = 0.0f;
+            for (int i = 0; i < 8; ++i) {
+                const int j = min(j0 + i * 4 + kq, end - 1);   // (a place past the end reads the last key and counts nothing)
+                const int page = j / page_size;
+                row[i] = pool + table[page] * page_elems + (int64_t)(j - page * page_size) * D + k_at;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float dot = 0.0f;
+#pragma unroll
+                for (int u = 0; u < PIECES; ++u) {
+                    const int d = sub * 4 + 32 * u;
+                    if (d < D) {
+                        const float4 k = *reinterpret_cast<const float4*>(row[i] + d);
+                        dot = fmaf(qv[u].x, k.x, dot);
+                        dot = fmaf(qv[u].y, k.y, dot);
+                        dot = fmaf(qv[u].z, k.z, dot);
+                        dot = fmaf(qv[u].w, k.w, dot);
+                    }
+                }
+                s[i] = dot;
+            }
+            float m_new = m;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
+                if (softcap > 0.0f) s[i] = softcap * tanhf(s[i] / softcap);
+                if (j0 + i * 4 + kq >= end) s[i] = -INFINITY;
+                m_new = fmaxf(m_new, s[i]);
+            }
+#pragma unroll
+            for (int o = 8; o < 32; o <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, o));
+            const float corr = expf(m - m_new);                // 0 on the warp's first block (m = -inf; a block has a key)
+            float sum = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                s[i] = j0 + i * 4 + kq < end ? expf(s[i] - m_new) : 0.0f;
+                sum += s[i];
+            }
+            l = l * corr + sum;                                // this lane's keys; the four groups are added at the end
+            m = m_new;
 #pragma unroll
             for (int u = 0; u < PIECES; ++u) {
-                const int d = sub * 4 + 32 * u;
-                if (d < D) {
-                    const float4 k = *reinterpret_cast<const float4*>(row[i] + d);
-                    dot = fmaf(qv[u].x, k.x, dot);
-                    dot = fmaf(qv[u].y, k.y, dot);
-                    dot = fmaf(qv[u].z, k.z, dot);
-                    dot = fmaf(qv[u].w, k.w, dot);
-                }
+                acc[u].x *= corr; acc[u].y *= corr; acc[u].z *= corr; acc[u].w *= corr;
             }
-            s[i] = dot;
-        }
-        float m_new = m;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < 8; ++i) {
+                const int j = min(j0 + i * 4 + kq, end - 1);
+                const int in_page = j % page_size;
+                const float* v = row[i] + (v_at - k_at) + (int64_t)in_page * (DV - D);
 #pragma unroll
-            for (int o = 1; o < 8; o <<= 1) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
-            if (softcap > 0.0f) s[i] = softcap * tanhf(s[i] / softcap);
-            if (j0 + i * 4 + kq >= end) s[i] = -INFINITY;
-            m_new = fmaxf(m_new, s[i]);
-        }
-#pragma unroll
-        for (int o = 8; o < 32; o <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, o));
-        const float corr = expf(m - m_new);                // 0 on the warp's first block (m = -inf; a block has a key)
-        float sum = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            s[i] = j0 + i * 4 + kq < end ? expf(s[i] - m_new) : 0.0f;
-            sum += s[i];
-        }
-        l = l * corr + sum;                                // this lane's keys; the four groups are added at the end
-        m = m_new;
-#pragma unroll
-        for (int u = 0; u < PIECES; ++u) {
-            acc[u].x *= corr; acc[u].y *= corr; acc[u].z *= corr; acc[u].w *= corr;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int j = min(j0 + i * 4 + kq, end - 1);
-            const int in_page = j % page_size;
-            const float* v = row[i] + (v_at - k_at) + (int64_t)in_page * (DV - D);
-#pragma unroll
-            for (int u = 0; u < PIECES; ++u) {
-                const int d = sub * 4 + 32 * u;
-                if (d < DV) {
-                    const float4 vv = *reinterpret_cast<const float4*>(v + d);
-                    acc[u].x = fmaf(s[i], vv.x, acc[u].x);
-                    acc[u].y = fmaf(s[i], vv.y, acc[u].y);
-                    acc[u].z = fmaf(s[i], vv.z, acc[u].z);
-                    acc[u].w = fmaf(s[i], vv.w, acc[u].w);
+                for (int u = 0; u < PIECES; ++u) {
+                    const int d = sub * 4 + 32 * u;
+                    if (d < DV) {
+                        const float4 vv = *reinterpret_cast<const float4*>(v + d);
+                        acc[u].x = fmaf(s[i], vv.x, acc[u].x);
+                        acc[u].y = fmaf(s[i], vv.y, acc[u].y);
+                        acc[u].z = fmaf(s[i], vv.z, acc[u].z);
+                        acc[u].w = fmaf(s[i], vv.w, acc[u].w);
+                    }
                 }
             }
         }
-    }
 #pragma unroll
-    for (int o = 8; o < 32; o <<= 1) {
-        l += __shfl_xor_sync(0xffffffffu, l, o);
-#pragma unroll
-        for (int u = 0; u < PIECES; ++u) {
-            acc[u].x += __shfl_xor_sync(0xffffffffu, acc[u].x, o);
-            acc[u].y += __shfl_xor_sync(0xffffffffu, acc[u].y, o);
-            acc[u].z += __shfl_xor_sync(0xffffffffu, acc[u].z, o);
-            acc[u].w += __shfl_xor_sync(0xffffffffu, acc[u].w, o);
-        }
-    }
-    float* maxima = merge_sm + warps * DV;
-    float* sums = maxima + warps;
-    if (kq == 0) {
+        for (int o = 8; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        // the four lanes of a channel add up, each of them a quarter of the channels that they share (half as many values a
+        // stage go out: 3 PIECES shuffles where sums in all four would take 8 PIECES)
+        float f[4 * PIECES];
 #pragma unroll
         for (int u = 0; u < PIECES; ++u) {
-            const int d = sub * 4 + 32 * u;
-            if (d < DV) *reinterpret_cast<float4*>(merge_sm + warp * DV + d) = acc[u];
+            f[4 * u] = acc[u].x; f[4 * u + 1] = acc[u].y; f[4 * u + 2] = acc[u].z; f[4 * u + 3] = acc[u].w;
         }
+#pragma unroll
+        for (int e = 0; e < 2 * PIECES; ++e) {
+            const float away = kq & 2 ? f[e] : f[e + 2 * PIECES], mine = kq & 2 ? f[e + 2 * PIECES] : f[e];
+            f[e] = mine + __shfl_xor_sync(0xffffffffu, away, 16);
+        }
+#pragma unroll
+        for (int e = 0; e < PIECES; ++e) {
+            const float away = kq & 1 ? f[e] : f[e + PIECES], mine = kq & 1 ? f[e + PIECES] : f[e];
+            f[e] = mine + __shfl_xor_sync(0xffffffffu, away, 8);
+        }
+        const int first = (kq & 2 ? 2 * PIECES : 0) + (kq & 1 ? PIECES : 0);
+#pragma unroll
+        for (int e = 0; e < PIECES; e += 2) {
+            const int d = sub * 4 + 32 * ((first + e) >> 2) + ((first + e) & 3);
+            if (d < DV) *reinterpret_cast<float2*>(merge_sm + group * DV + d) = make_float2(f[e], f[e + 1]);
+        }
+        if (lane == 0) { maxima[group] = m; sums[group] = l; }
     }
-    if (lane == 0) { maxima[warp] = m; sums[warp] = l; }
     __syncthreads();
     float top = plus_one ? 0.0f : -INFINITY;
-    for (int w = 0; w < warps; ++w) top = fmaxf(top, maxima[w]);
+    for (int w = 0; w < used; ++w) top = fmaxf(top, maxima[w]);
+    if ((int)threadIdx.x < used) weights[threadIdx.x] = expf(maxima[threadIdx.x] - top);
+    __syncthreads();
     float den = plus_one ? expf(0.0f - top) : 0.0f;
-    for (int w = 0; w < warps; ++w) den += sums[w] * expf(maxima[w] - top);    // (a warp without blocks: -inf, 0)
+    for (int w = 0; w < used; ++w) den += sums[w] * weights[w];
     float g = 1.0f;
     if (gate != nullptr && !gate_channels) g = 1.0f / (1.0f + expf(-gate[(int64_t)t * ld_gate + h]));
     const float norm = g / den;
     for (int d = threadIdx.x; d < DV; d += blockDim.x) {
         float v = 0.0f;
-        for (int w = 0; w < warps; ++w) v = fmaf(merge_sm[w * DV + d], expf(maxima[w] - top), v);
+        for (int w = 0; w < used; ++w) v = fmaf(merge_sm[w * DV + d], weights[w], v);
         v *= norm;
         if (gate != nullptr && gate_channels) v *= 1.0f / (1.0f + expf(-gate[(int64_t)t * ld_gate + h * DV + d]));
         out[(int64_t)t * ld_out + (int64_t)h * DV + d] = v;
@@ -527,10 +549,11 @@ XS_API int xs_attention_generic(const void* q, const void* pool, const int32_t* 
     XS_REQUIRE(page_size > 0 && P > 0 && keep >= 0, "attention: window %d, page size %d, %d pages", window, page_size, P);
     const int most = D > DV ? D : DV;
     if (dtype == XS_F32 && D % 4 == 0 && DV % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)pool % 16 == 0 && (int64_t)T * Hq < 2147483647) {
-        // few (token, head) pairs: many warps each, so that a decode step's keys are read by the whole device
-        // (16 warps of the 64-channel instance, 8 of the wider ones fit a CTA's registers)
-        const int per = (int64_t)T * Hq > 4 * 148 ? 4 : most <= 64 ? 16 : 8;
-        const size_t bytes = (size_t)per * (DV + 2) * sizeof(float);
+        // few (token, head) pairs: a warp a group, so that a decode step's keys are read by the whole device; many: four warps
+        // that take the groups in turn, so that more CTAs fit an SM
+        const int groups = most <= 64 ? kAttnF32Groups<2> : kAttnF32Groups<4>;
+        const int per = (int64_t)T * Hq > 4 * 148 ? 4 : groups;
+        const size_t bytes = (size_t)groups * (DV + 3) * sizeof(float);
 #define XS_ATTN_F32(PC)                                                                                                              \
     xs_launch(attention_f32_kernel<PC>, dim3(T * Hq), dim3(per * 32), bytes, stream, (const float*)q, (const float*)pool, page_table, \
               P, seq_of_token, positions, (const float*)gate, ld_gate, (float*)out, ld_out, Hq, Hkv, D, DV, planes, page_size,        \
