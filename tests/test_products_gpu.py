@@ -122,6 +122,45 @@ def test_float32_attention_does_not_depend_on_the_step(H, G, D, DV, window, keep
     assert torch.equal(attend(77, 1)[0], attend(0, T)[77])
 
 
+@pytest.mark.parametrize("plus", [0, 1])
+@pytest.mark.parametrize("keys", [5, 64, 90, 600])
+def test_float32_attention_of_values_that_are_not_finite(plus, keys):
+    """Against the kernel of other alignments: an infinite value of the last key, keys whose scores are minus infinity."""
+    H, D, page, P = 2, 64, 64, 10
+    pool = torch.randn(P, 2, H, page, D, device=DEV)
+    pages, seq = torch.arange(P, dtype=torch.int32, device=DEV).view(1, P), torch.zeros(1, dtype=torch.int32, device=DEV)
+    pos = torch.tensor([keys - 1], dtype=torch.int32, device=DEV)
+    flat_q = torch.randn(H * D + 1, device=DEV)
+    flat_q[::8] = flat_q[::8].abs() + 0.1
+    flat_q[1:] = flat_q[:-1].clone()
+
+    def both():
+        res = []
+        for off in (0, 1):                # (the second on an odd word: the general kernel)
+            q = flat_q.clone()[1:].clone() if off == 0 else flat_q[1:]
+            out = torch.empty(1, H, D, device=DEV)
+            ops()._check(ops().load().xs_attention_generic(
+                q.data_ptr(), pool.data_ptr(), pages.data_ptr(), P, seq.data_ptr(), pos.data_ptr(), None, 0, out.data_ptr(), H * D, 1, H, H, D,
+                D, 2, page, D ** -0.5, 0.0, 0, 0, plus, 0, 0, ops()._stream()))
+            res.append(out)
+        return res
+
+    pool[(keys - 1) // page, 1, :, (keys - 1) % page, 7] = math.inf
+    got, want = both()
+    assert bool((want[..., 7] == math.inf).all()) and torch.equal(got.isinf(), want.isinf())
+    fine = torch.isfinite(want)
+    assert (got[fine] - want[fine]).abs().max() <= 4e-6 * want[fine].abs().max()
+    if keys > 64 or plus:
+        # (only the keys behind position 31 where the denominator has no term of its own, so that the general kernel's first block has a maximum)
+        pool[:, 1].clamp_(-9.0, 9.0)
+        first = 0 if plus else 32
+        hidden = torch.arange(P * page, device=DEV).view(P, page)
+        pool[:, 0, :, :, 0] = torch.where(((hidden >= first) & (hidden < 64))[:, None], torch.tensor(-math.inf, device=DEV), pool[:, 0, :, :, 0])
+        got, want = both()
+        assert torch.isfinite(want).all() and torch.isfinite(got).all()
+        assert (got - want).abs().max() <= 4e-6 * want.abs().max().clamp(min=1e-6)
+
+
 # --------------------------------------------------------------------------- tcgen05 product, many tokens: the store paths
 @pytest.mark.parametrize("T,N", [(65, 48), (128, 272), (129, 256), (300, 528), (1000, 80)])
 @pytest.mark.parametrize("pad", [0, 8, 1])

@@ -8,6 +8,9 @@
 // pos sees key j iff j <= pos and (window == 0 or pos - j < window or j < keep)
 // (src/backend/cpu_ref/ops.cpp:567-571; keep: a window's kept first positions); head h reads
 // kv head h / (heads / kv_heads) (ops.cpp:588). Scores, softmax and the weighted sum are float32.
+#include <float.h>
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -368,79 +371,93 @@ __global__ void attention_f32_kernel(const float* __restrict__ q, const float* _
     float* weights = sums + G;
     for (int group = warp; group < used; group += warps) {
         float4 acc[PIECES];
+        float m, l;
+        auto walk = [&](auto careful) {
+            constexpr bool kCareful = decltype(careful)::value;
 #pragma unroll
-        for (int u = 0; u < PIECES; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        float m = -INFINITY, l = 0.0f;
-        for (int b = group; b < blocks; b += G) {
-            const bool early = b < kept_blocks;
-            const int j0 = early ? b * 32 : lo + (b - kept_blocks) * 32;
-            const int end = early ? kept : pos + 1;
-            const float* row[8];
-            float s[8];
+            for (int u = 0; u < PIECES; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            // (the lowest finite number, not minus infinity: a first block whose scores are all minus infinity then counts nothing)
+            m = -FLT_MAX;
+            l = 0.0f;
+            for (int b = group; b < blocks; b += G) {
+                const bool early = b < kept_blocks;
+                const int j0 = early ? b * 32 : lo + (b - kept_blocks) * 32;
+                const int end = early ? kept : pos + 1;
+                const float* row[8];
+                float s[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int j = min(j0 + i * 4 + kq, end - 1);   // (a place past the end reads the last key and counts nothing)
-                const int page = j / page_size;
-                row[i] = pool + table[page] * page_elems + (int64_t)(j - page * page_size) * D + k_at;
-            }
+                for (int i = 0; i < 8; ++i) {
+                    const int j = min(j0 + i * 4 + kq, end - 1);   // (a place past the end reads the last key and counts nothing)
+                    const int page = j / page_size;
+                    row[i] = pool + table[page] * page_elems + (int64_t)(j - page * page_size) * D + k_at;
+                }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                float dot = 0.0f;
+                for (int i = 0; i < 8; ++i) {
+                    float dot = 0.0f;
+#pragma unroll
+                    for (int u = 0; u < PIECES; ++u) {
+                        const int d = sub * 4 + 32 * u;
+                        if (d < D) {
+                            const float4 k = *reinterpret_cast<const float4*>(row[i] + d);
+                            dot = fmaf(qv[u].x, k.x, dot);
+                            dot = fmaf(qv[u].y, k.y, dot);
+                            dot = fmaf(qv[u].z, k.z, dot);
+                            dot = fmaf(qv[u].w, k.w, dot);
+                        }
+                    }
+                    s[i] = dot;
+                }
+                float m_new = m;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+#pragma unroll
+                    for (int o = 1; o < 8; o <<= 1) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
+                    if (softcap > 0.0f) s[i] = softcap * tanhf(s[i] / softcap);
+                    if (j0 + i * 4 + kq >= end) s[i] = -INFINITY;
+                    m_new = fmaxf(m_new, s[i]);
+                }
+#pragma unroll
+                for (int o = 8; o < 32; o <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, o));
+                const float corr = expf(m - m_new);                // 0 on the warp's first block (m = -inf; a block has a key)
+                float sum = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    s[i] = j0 + i * 4 + kq < end ? expf(s[i] - m_new) : 0.0f;
+                    sum += s[i];
+                }
+                l = l * corr + sum;                                // this lane's keys; the four groups are added at the end
+                m = m_new;
 #pragma unroll
                 for (int u = 0; u < PIECES; ++u) {
-                    const int d = sub * 4 + 32 * u;
-                    if (d < D) {
-                        const float4 k = *reinterpret_cast<const float4*>(row[i] + d);
-                        dot = fmaf(qv[u].x, k.x, dot);
-                        dot = fmaf(qv[u].y, k.y, dot);
-                        dot = fmaf(qv[u].z, k.z, dot);
-                        dot = fmaf(qv[u].w, k.w, dot);
-                    }
+                    acc[u].x *= corr; acc[u].y *= corr; acc[u].z *= corr; acc[u].w *= corr;
                 }
-                s[i] = dot;
-            }
-            float m_new = m;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 8; ++i) {
+                    const int j = min(j0 + i * 4 + kq, end - 1);
+                    const int in_page = j % page_size;
+                    const float* v = row[i] + (v_at - k_at) + (int64_t)in_page * (DV - D);
 #pragma unroll
-                for (int o = 1; o < 8; o <<= 1) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
-                if (softcap > 0.0f) s[i] = softcap * tanhf(s[i] / softcap);
-                if (j0 + i * 4 + kq >= end) s[i] = -INFINITY;
-                m_new = fmaxf(m_new, s[i]);
-            }
-#pragma unroll
-            for (int o = 8; o < 32; o <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, o));
-            const float corr = expf(m - m_new);                // 0 on the warp's first block (m = -inf; a block has a key)
-            float sum = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                s[i] = j0 + i * 4 + kq < end ? expf(s[i] - m_new) : 0.0f;
-                sum += s[i];
-            }
-            l = l * corr + sum;                                // this lane's keys; the four groups are added at the end
-            m = m_new;
-#pragma unroll
-            for (int u = 0; u < PIECES; ++u) {
-                acc[u].x *= corr; acc[u].y *= corr; acc[u].z *= corr; acc[u].w *= corr;
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int j = min(j0 + i * 4 + kq, end - 1);
-                const int in_page = j % page_size;
-                const float* v = row[i] + (v_at - k_at) + (int64_t)in_page * (DV - D);
-#pragma unroll
-                for (int u = 0; u < PIECES; ++u) {
-                    const int d = sub * 4 + 32 * u;
-                    if (d < DV) {
-                        const float4 vv = *reinterpret_cast<const float4*>(v + d);
-                        acc[u].x = fmaf(s[i], vv.x, acc[u].x);
-                        acc[u].y = fmaf(s[i], vv.y, acc[u].y);
-                        acc[u].z = fmaf(s[i], vv.z, acc[u].z);
-                        acc[u].w = fmaf(s[i], vv.w, acc[u].w);
+                    for (int u = 0; u < PIECES; ++u) {
+                        const int d = sub * 4 + 32 * u;
+                        if (d < DV) {
+                            float4 vv = *reinterpret_cast<const float4*>(v + d);
+                            if (kCareful && j0 + i * 4 + kq >= end) vv = make_float4(0.f, 0.f, 0.f, 0.f);
+                            acc[u].x = fmaf(s[i], vv.x, acc[u].x);
+                            acc[u].y = fmaf(s[i], vv.y, acc[u].y);
+                            acc[u].z = fmaf(s[i], vv.z, acc[u].z);
+                            acc[u].w = fmaf(s[i], vv.w, acc[u].w);
+                        }
                     }
                 }
             }
-        }
+        };
+        walk(std::false_type{});
+        // A place past the end added 0 times the last key's value, which is not 0 where that is not finite. A test in every block
+        // costs 5 to 20 %; so the walk is done again, with it, where an output is not finite.
+        float odd = 0.0f;
+#pragma unroll
+        for (int u = 0; u < PIECES; ++u) odd += 0.0f * acc[u].x + 0.0f * acc[u].y + 0.0f * acc[u].z + 0.0f * acc[u].w;
+        if (__any_sync(0xffffffffu, !(odd == 0.0f))) walk(std::true_type{});
 #pragma unroll
         for (int o = 8; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
         // the four lanes of a channel add up, each of them a quarter of the channels that they share (half as many values a
