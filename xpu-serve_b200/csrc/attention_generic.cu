@@ -336,12 +336,13 @@ template <int PIECES>
 constexpr int kAttnF32Groups = PIECES <= 2 ? 16 : 8;
 
 template <int PIECES>
-__global__ void attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ pool,
-                                     const int32_t* __restrict__ page_table, int P, const int32_t* __restrict__ seq_of_token,
-                                     const int32_t* __restrict__ positions, const float* __restrict__ gate, int64_t ld_gate,
-                                     float* __restrict__ out, int64_t ld_out, int Hq, int Hkv, int D, int DV, int planes,
-                                     int page_size, float scale, float softcap, int window, int keep, int plus_one,
-                                     int gate_channels) {
+__global__ void __launch_bounds__(32 * kAttnF32Groups<PIECES>)      // (a warp a group at most)
+attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ pool,
+                     const int32_t* __restrict__ page_table, int P, const int32_t* __restrict__ seq_of_token,
+                     const int32_t* __restrict__ positions, const float* __restrict__ gate, int64_t ld_gate,
+                     float* __restrict__ out, int64_t ld_out, int Hq, int Hkv, int D, int DV, int planes,
+                     int page_size, float scale, float softcap, int window, int keep, int plus_one,
+                     int gate_channels) {
     constexpr int G = kAttnF32Groups<PIECES>;
     extern __shared__ __align__(16) float merge_sm[];     // [G][DV] outputs, then [G] maxima, [G] sums, [G] weights
     pdl_launch_dependents();
