@@ -273,6 +273,51 @@ def test_experts_of_few_tokens(T, top, E, F, H, act):
     assert gap(y, (rows * wts.double()[:, None]).view(T, top, H).sum(1)) <= 2.0 ** -8
 
 
+@pytest.mark.parametrize("E,top", [(5, 5), (9, 3), (40, 8), (64, 2), (130, 6), (256, 16), (300, 4)])
+@pytest.mark.parametrize("router", ["top", "sigmoid", "softmax", "groups"])
+def test_choices_are_experts_and_differ(E, top, router):
+    """Whatever the logits are: NaN, infinite, equal."""
+    inf, nan = math.inf, math.nan
+    rows = [torch.full((E,), nan), torch.full((E,), -inf), torch.full((E,), inf), torch.zeros(E), torch.randn(E), torch.randn(E), torch.randn(E)]
+    rows[4][::2] = nan
+    rows[5][1:] = -inf
+    rows[6][: E - 1] = nan
+    rows += [torch.randn(E) for _ in range(8 - len(rows))]
+    logits = torch.stack(rows).to(DEV)
+    T = logits.shape[0]
+    ids = torch.full((T * top,), 12345, dtype=torch.int32, device=DEV)
+    wts = torch.empty(T * top, device=DEV)
+    if router == "top":
+        ops().moe_route(logits, top, ids, wts)
+    else:
+        groups = next(g for g in (4, 3, 2, 1) if E % g == 0) if router == "groups" else 1
+        keep = next(k for k in range(1, groups + 1) if k * (E // groups) >= top)
+        ops().moe_route_grouped(logits, top, ids, wts, experts=E, score="softmax" if router == "softmax" else "sigmoid",
+                                groups=groups, keep=keep, group_top=2, renorm=True, renorm_eps=0.0)
+    got = ids.view(T, top).tolist()
+    for t, choices in enumerate(got):
+        assert all(0 <= e < E for e in choices) and len(set(choices)) == top, (t, choices)
+    assert torch.isnan(wts.view(T, top)[0]).all()      # a token of NaNs stays one
+    want = torch.topk(logits[7], top).indices.tolist()
+    assert router == "groups" or got[7] == want
+
+
+def test_a_token_of_nan_leaves_the_others_alone():
+    T, top, E, F, H = 8, 8, 16, 40, 264
+    x, w = torch.randn(T, H, device=DEV).to(BF), torch.randn(E, F, H, device=DEV).to(BF)
+    logits = torch.randn(T, E, device=DEV)
+    logits[:, 0] = 9.0                 # everybody names expert 0
+    logits[0] = math.nan
+    ids, wts = torch.empty(T * top, dtype=torch.int32, device=DEV), torch.empty(T * top, device=DEV)
+    ops().moe_route_grouped(logits, top, ids, wts, experts=E)
+    out = torch.full((T * top, F), math.nan, device=DEV, dtype=BF)
+    ops().moe_few_rows(x, top, w, out, ids, T, glu=False)
+    ref = torch.einsum("tkfh,th->tkf", w.double()[ids.view(T, top).long()], x.double()).reshape(T * top, F)
+    assert gap(out, ref) <= 2.0 ** -8
+    with pytest.raises(ops().KernelError, match="choices"):
+        ops().moe_few_rows(x, top, w, out, ids, 7, glu=False)
+
+
 @pytest.mark.parametrize("M,F,K", [(1, 8, 8), (3, 24, 264), (8, 1024, 2048), (8, 16, 8192), (9, 40, 1032), (16, 1024, 2048)])
 @pytest.mark.parametrize("slices", [1, 4])
 def test_clamped_unit_of_few_rows(M, F, K, slices):

@@ -176,6 +176,11 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, int ld, int T
     }
 }
 
+// Every routing kernel names experts that differ, whatever the logits are: the products of few tokens count on it, and the plan on
+// choices that are experts. Where only NaNs and minus infinities are left the warp kernels choose by index (a branch that costs a
+// comparison a choice: what is taken is told from what is minus infinity only there).
+constexpr int kNaNsBehind = 1 << 28;
+
 // A warp per token (E <= 256): a lane holds logits lane, lane + 32, ...; each of the `top` rounds finds the largest logit
 // left (ties: the lower index) by a reduction over the warp.
 __global__ void moe_route_warp_kernel(const float* __restrict__ logits, int ld, int T, int E, int top, float scale,
@@ -191,6 +196,7 @@ __global__ void moe_route_warp_kernel(const float* __restrict__ logits, int ld, 
     for (int j = 0; j < 8; ++j) v[j] = lane + 32 * j < E ? z[lane + 32 * j] : -INFINITY;
     float mine = 0.0f, largest = 0.0f, sum = 0.0f;
     int mine_id = 0;
+    unsigned taken = 0;                 // of this lane's eight
     for (int k = 0; k < top; ++k) {
         float bv = -INFINITY;
         int bi = 1 << 30;
@@ -211,9 +217,26 @@ __global__ void moe_route_warp_kernel(const float* __restrict__ logits, int ld, 
                 bi = oi;
             }
         }
+        if (!(bv > -INFINITY)) {        // nothing above minus infinity is left: the lowest index not taken, NaNs behind it
+            bi = kNaNsBehind << 1;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int e = lane + 32 * j;
+                if (e < E && !(taken >> j & 1u)) bi = min(bi, v[j] == v[j] ? e : e + kNaNsBehind);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) bi = min(bi, __shfl_xor_sync(0xffffffffu, bi, o));
+            if (bi >= kNaNsBehind) {
+                bi -= kNaNsBehind;
+                bv = NAN;
+            }
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            if (lane + 32 * j == bi) v[j] = -INFINITY;       // taken (a logit of -inf itself is never chosen twice: its index is)
+            if (lane + 32 * j == bi) {
+                v[j] = -INFINITY;
+                taken |= 1u << j;
+            }
         if (k == 0) largest = bv;
         const float p = expf(bv - largest);
         sum += p;
@@ -238,6 +261,7 @@ __global__ void moe_route_warp_kernel(const float* __restrict__ logits, int ld, 
 // output is their input): a choice of one is written as id -1, with its weight.
 // `squared`: the weights' squares are written (experts that are homogeneous of degree two, fed their weight times the input).
 // A warp per token; the token's s and c stand in shared memory (2 E floats a warp).
+constexpr float kTaken = -1.0f;                 // in place of a chosen expert's s (scores are 0 to 1)
 __global__ void moe_route_grouped_kernel(const float* __restrict__ logits, int ld, int T, int E, int top,
                                          const float* __restrict__ correction, int groups, int keep, int group_top, float scale,
                                          int renorm, float renorm_eps, int squared, int score, int real, int32_t* __restrict__ ids,
@@ -321,10 +345,20 @@ __global__ void moe_route_grouped_kernel(const float* __restrict__ logits, int l
                 bi = oi;
             }
         }
-        if (bi >= E) bi = 0;                    // (only a row of NaNs comes here)
+        if (!(bv > -INFINITY)) {                // nothing above minus infinity is left: the lowest index not taken, NaNs behind it
+            bi = kNaNsBehind << 1;
+            for (int e = lane; e < E; e += 32)
+                if (s[e] != kTaken) bi = min(bi, c[e] == c[e] ? e : e + kNaNsBehind);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) bi = min(bi, __shfl_xor_sync(0xffffffffu, bi, o));
+            bi &= kNaNsBehind - 1;
+        }
         const float w = s[bi];
         __syncwarp();
-        if (lane == 0) c[bi] = -INFINITY;       // taken (enough experts are open, so none at minus infinity is ever chosen)
+        if (lane == 0) {
+            c[bi] = -INFINITY;                  // taken
+            s[bi] = kTaken;
+        }
         __syncwarp();
         sum += w;
         if (lane == k) {

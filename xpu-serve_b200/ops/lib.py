@@ -1116,13 +1116,16 @@ MOE_FEW_TOKENS = 32      # the most tokens `moe_few_rows` takes (an expert then 
 def moe_few_rows(x: torch.Tensor, share: int, w: torch.Tensor, out: torch.Tensor, ids: torch.Tensor, tokens: int, glu: bool,
                  clamp=None, relu_squared: bool = False) -> None:
     """out[i] = w[ids[i]] . x[i // share] for the rows i of a step's choices in the router's own order (rows whose id is -1 are
-    left alone), `tokens` at most MOE_FEW_TOKENS. w, `glu`, `clamp` and `relu_squared` as in gemm_tc_grouped."""
+    left alone), `tokens` at most MOE_FEW_TOKENS. A token names an expert at most once, as the routing kernels see to: an expert
+    has at most `tokens` rows. w, `glu`, `clamp` and `relu_squared` as in gemm_tc_grouped."""
     limit, alpha, shift = (0.0, 1.0, 0.0) if clamp is None else clamp
     if glu and relu_squared:
         raise KernelError("moe_few_rows: one activation at a time")
     _need(w, "expert weights", torch.bfloat16); _need(ids, "ids", torch.int32)
     E, N, K = w.shape
     rows = ids.numel()
+    if tokens < 1 or rows % tokens != 0:
+        raise KernelError(f"moe_few_rows: {rows} rows are not {tokens} tokens' choices")
     for t, name in ((x, "x"), (out, "out")):
         if not t.is_cuda or t.dtype != torch.bfloat16 or t.dim() != 2 or t.stride(1) != 1:
             raise KernelError(f"moe_few_rows: {name} must be a bfloat16 CUDA matrix with contiguous rows")
