@@ -68,3 +68,11 @@ def test_every_cache_has_a_serial_number_of_its_own():
         assert c.serial not in seen
         seen.add(c.serial)
         del c                                          # the next one may get the same id(), never the same serial
+
+
+def test_tokens_up_to_which_experts_take_the_product_of_few_rows():
+    """16 in general, 32 where the two products have at most 1,024 CTAs of 32 weight rows."""
+    from xpu_serve_b200.ops import lib
+    assert lib.moe_few_tokens(16, 2 * 1024, 2048) == 16 and lib.moe_few_tokens(64, 2 * 512, 2048) == 16
+    assert lib.moe_few_tokens(8, 2 * 256, 512) == 32 and lib.moe_few_tokens(16, 2 * 512, 1024) == 32
+    assert lib.moe_few_tokens(16, 2 * 512, 1025) == 16 and lib.moe_few_tokens(1, 8, 8) == lib.MOE_FEW_TOKENS

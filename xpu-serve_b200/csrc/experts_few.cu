@@ -11,8 +11,9 @@
 //     the order of the warps. A row's result does not depend on the other rows of the step.
 // Bound by the weights' bytes of the experts that are met. Measured on B200 (8 tokens, top 4 of 16 experts of 1,024 at width 2,048:
 // 177 MB of weights, kernels alone): gate/up and down 35 + 20 us (3.2 TB/s, cold), where gather, two tcgen05 products over padded
-// tiles of 128 rows and the plan took 120; a decode step of four such layers 0.69 -> 0.63 ms. From 33 tokens on the tiles are at
-// least a quarter full and the tcgen05 products take over.
+// tiles of 128 rows and the plan took 120; a decode step of four such layers 0.69 -> 0.63 ms. A product's time follows the
+// groups of eight columns that it carries, whatever an expert's count is: the tcgen05 products take over at 17 tokens, or at 33 for
+// small experts (ops/lib.py moe_few_tokens has both sides; 32 rows an expert are the most that an instance here holds).
 #include "common.cuh"
 #include "few_rows.cuh"
 

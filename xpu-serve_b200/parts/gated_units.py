@@ -162,6 +162,7 @@ class RoutedExperts(FeedForward):
 
         self.w_gate_up = rt.matrix(torch.stack([stacked(e) for e in range(spec.experts)]))
         self.w_down = rt.matrix(torch.stack([weights[n["down"].format(e=e)].to(torch.float32) for e in range(spec.experts)]))
+        self.few_tokens = ops.moe_few_tokens(spec.experts, self.w_gate_up.shape[1], H) if self.tensor_cores else 0
         router = weights[n["router"]].to(torch.float32)
         self.shared = None
         if spec.shared is not None:
@@ -199,7 +200,7 @@ class RoutedExperts(FeedForward):
             ops.moe_route(logits, s.top, ids, wts, experts=s.experts, scale=s.route_scale)
         out = ws.get("ffn_out", (T, s.hidden), rt.act_dtype)
         passed = {"passed": y} if self.identity else {}       # (choices that stand for the token's input itself)
-        if self.tensor_cores and T <= ops.MOE_FEW_TOKENS:
+        if T <= self.few_tokens:
             # few tokens: the products find each expert's rows in the router's ids, which stay in their order (csrc/experts_few.cu)
             act = ws.get("moe_act_few", (n, s.intermediate), rt.act_dtype)
             ops.moe_few_rows(y, s.top, self.w_gate_up, act, ids, T, glu=self.gated, clamp=self.clamp, relu_squared=not self.gated)
