@@ -76,3 +76,47 @@ def test_tokens_up_to_which_experts_take_the_product_of_few_rows():
     assert lib.moe_few_tokens(16, 2 * 1024, 2048) == 16 and lib.moe_few_tokens(64, 2 * 512, 2048) == 16
     assert lib.moe_few_tokens(8, 2 * 256, 512) == 32 and lib.moe_few_tokens(16, 2 * 512, 1024) == 32
     assert lib.moe_few_tokens(16, 2 * 512, 1025) == 16 and lib.moe_few_tokens(1, 8, 8) == lib.MOE_FEW_TOKENS
+
+
+class _RecordedOps:
+    """Stands for the kernels: remembers which ran."""
+
+    def __init__(self, real):
+        self.real, self.ran = real, []
+
+    def __getattr__(self, name):
+        if name in ("moe_few_tokens", "MOE_FEW_TOKENS"):
+            return getattr(self.real, name)
+        if name.startswith("moe_max_tiles"):
+            return lambda rows, experts, tile_rows=64: rows // tile_rows + min(rows, experts)
+        return lambda *a, **k: self.ran.append(name)
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 17])
+def test_experts_take_the_buffers_of_their_own_route(tokens, monkeypatch):
+    """A step whose products find the experts' rows by themselves keeps no plan (each captured decode step would hold one)."""
+    from types import SimpleNamespace
+
+    from xpu_serve_b200.config.spec import RoutedExpertsSpec
+    from xpu_serve_b200.parts import gated_units
+    E, F, H = 64, 64, 512
+    names = {"gate": "g{e}", "up": "u{e}", "down": "d{e}", "router": "r"}
+    spec = RoutedExpertsSpec(hidden=H, intermediate=F, experts=E, top=2, names=names)
+    weights = {"r": torch.zeros(E, H)}
+    for e in range(E):
+        weights.update({f"g{e}": torch.zeros(F, H), f"u{e}": torch.zeros(F, H), f"d{e}": torch.zeros(H, F)})
+    ops = _RecordedOps(gated_units.ops)
+    monkeypatch.setattr(gated_units, "ops", ops)
+    rt = SimpleNamespace(mode="bfloat16", act_dtype=torch.bfloat16, ws=Workspace(torch.device("cpu")),
+                         matrix=lambda t: t.to(torch.bfloat16), vector=lambda t: t)
+    unit = gated_units.RoutedExperts(spec, weights, rt)
+    assert unit.few_tokens == 16
+    unit.forward(torch.zeros(tokens, H, dtype=torch.bfloat16), None)
+    kept = {name for name, _ in rt.ws._bufs if name.startswith("moe_")}
+    if tokens <= 16:
+        assert "moe_few_rows" in ops.ran and "moe_plan" not in ops.ran
+        assert kept == {"moe_logits", "moe_ids", "moe_wts", "moe_act_few", "moe_rows_few"}
+    else:
+        assert "moe_plan" in ops.ran and "moe_few_rows" not in ops.ran
+        assert kept == {"moe_logits", "moe_ids", "moe_wts", "moe_place", "moe_source_padded", "moe_meta_padded", "moe_rows_in",
+                        "moe_act", "moe_rows"}

@@ -185,9 +185,6 @@ class RoutedExperts(FeedForward):
         shared_gate = logits[:, outputs:] if shared is not None and s.shared_gated else None
         ids = ws.get("moe_ids", (n,), torch.int32)
         wts = ws.get("moe_wts", (n,), torch.float32)
-        place = ws.get("moe_place", (n,), torch.int32)
-        source = ws.get("moe_source", (n,), torch.int32)
-        meta = ws.get("moe_meta", (4 + 3 * ops.moe_max_tiles(n, s.experts),), torch.int32)
         if s.score == "softmax_all":
             ops.moe_route_grouped(logits, s.top, ids, wts, experts=outputs, correction=self.correction, scale=s.route_scale,
                                   score="softmax", real=s.experts, groups=s.groups, keep=s.keep_groups,
@@ -208,6 +205,7 @@ class RoutedExperts(FeedForward):
             ops.moe_few_rows(act, 1, self.w_down, rows_out, ids, T, glu=False)
             ops.moe_combine(rows_out, ids, wts, out, s.top, shared, shared_gate, in_place=True, **passed)
             return out
+        place = ws.get("moe_place", (n,), torch.int32)
         if self.tensor_cores:
             # every expert's rows padded to tiles of 128: gather, two tcgen05 products over the plan's tiles, combine
             tiles = ops.moe_max_tiles_of(n, s.experts, 128)
@@ -223,6 +221,8 @@ class RoutedExperts(FeedForward):
             ops.gemm_tc_grouped(act, self.w_down, rows_out, meta, tiles, glu=False)
             ops.moe_combine(rows_out, place, wts, out, s.top, shared, shared_gate, **passed)
             return out
+        source = ws.get("moe_source", (n,), torch.int32)
+        meta = ws.get("moe_meta", (4 + 3 * ops.moe_max_tiles(n, s.experts),), torch.int32)
         ops.moe_plan(ids, s.experts, place, source, meta)
         act = ws.get("moe_act", (n, s.intermediate), rt.act_dtype)
         ops.moe_gemm(y, self.w_gate_up, act, meta, n, source, s.top, glu=self.gated, clamp=self.clamp)
