@@ -374,7 +374,8 @@ def test_grouped_norm(groups, part, act, dtype):
     assert gap(y, ref) <= (2.0 ** -8 if dtype == BF else 2e-6)
 
 
-@pytest.mark.parametrize("heads,P,N,G,seqs", [(4, 4, 1, 2, 1), (6, 64, 128, 3, 8), (2, 20, 37, 1, 3), (3, 132, 300, 3, 2), (2, 1024, 16, 1, 1)])
+@pytest.mark.parametrize("heads,P,N,G,seqs", [(4, 4, 1, 2, 1), (6, 64, 128, 3, 8), (2, 20, 37, 1, 3), (3, 132, 300, 3, 2), (2, 1024, 16, 1, 1),
+                                              (2, 7, 301, 1, 2)])
 @pytest.mark.parametrize("dtype", [torch.float32, BF])
 def test_mamba2_step(heads, P, N, G, seqs, dtype):
     inner = heads * P
@@ -395,6 +396,25 @@ def test_mamba2_step(heads, P, N, G, seqs, dtype):
     assert gap(y, want) <= 4e-6 and gap(state[slots.long()], s) <= 2e-6
     rest = torch.tensor([i for i in range(seqs + 2) if i not in set(slots.tolist())], device=DEV)
     assert torch.equal(state[rest], state0[rest])
+
+
+@pytest.mark.parametrize("heads,P,N,G,seqs", [(4, 4, 4, 2, 1), (6, 64, 128, 3, 8), (2, 20, 36, 1, 3), (3, 132, 200, 3, 2), (2, 256, 16, 1, 1),
+                                              (4, 30, 200, 4, 5), (2, 260, 64, 1, 2), (2, 20, 37, 1, 3), (2, 33, 150, 2, 2), (4, 3, 1, 2, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_mamba2_step_is_the_scan_of_one_token(heads, P, N, G, seqs, dtype):
+    """A token's outputs and state do not depend on whether its step holds single tokens only: the same bits."""
+    inner = heads * P
+    C = inner + 2 * G * N
+    r = lambda *s: torch.randn(*s, device=DEV)                                     # noqa: E731
+    xbc, proj = r(seqs, C).to(dtype), r(seqs, inner + C + heads).to(dtype)
+    bias, a_log, skip, state = r(heads), r(heads) * 0.5, r(heads), r(seqs, heads, N, P)
+    slots, cu = torch.arange(seqs, dtype=torch.int32, device=DEV), torch.arange(seqs + 1, dtype=torch.int32, device=DEV)
+    got = []
+    for single in (True, False):
+        s, y = state.clone(), torch.empty(seqs, inner, device=DEV)
+        ops().mamba2_scan(xbc, proj, inner + C, bias, a_log, skip, s, cu, slots, y, heads, P, N, G, single=single)
+        got.append((s, y))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
 @pytest.mark.parametrize("taps,C,col0,seqs", [(1, 16, 8, 2), (2, 24, 0, 1), (3, 1032, 16, 5), (4, 64, 8, 8), (5, 48, 8, 3), (4, 20, 4, 3)])

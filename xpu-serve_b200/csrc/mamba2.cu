@@ -333,75 +333,83 @@ __global__ void mamba2_scan_kernel(ScanArgs a) {
     }
 }
 
-// One token a sequence (a decode step): a CTA per (head, sequence) of 256 threads. A thread holds four neighbouring columns of
-// every `rows`-th row of the state (16-byte loads, eight of them in flight), so that the state streams through the whole CTA;
-// the rows' shares of y meet in shared memory and are added in the order of the threads' rows. Bound by the state's bytes, read
-// and written once; the kernel above keeps a column a thread (two warps a CTA at 64 columns, 4-byte loads, all rows in registers),
-// which is made for many tokens. Measured on B200 (8 sequences, 64 heads, a 128 x 64 state: 34 MB): 11.4 us, 22.6 there.
-template <typename T>
-__global__ void __launch_bounds__(256) mamba2_step_kernel(ScanArgs a) {
-    __shared__ __align__(16) float part[256 * 4];
+// One token a sequence (a decode step): a CTA per (head, sequence, 128 columns). Where N is a multiple of 4 thread (j, p) takes the rows
+// j, j + 4, j + 8, ... of column p (WAYS 4), else all of them (WAYS 1), up to 32 loads in flight, asked for before the step size is known
+// (a warp issues in order). Those are the sums of the kernel above, which keeps a column a thread and, for such N, four sums of every
+// fourth row: a token's outputs are the same bits whether its step holds single tokens only or a longer piece beside it. Bound by the
+// state's bytes, read and written once. Measured on B200 (64 heads, a 128 x 64 state, bfloat16, L2
+// flushed, launch included): 8 sequences 15.1 us (17.4 by the kernel above, 16.4 by a form that summed in an order of its own), 32
+// sequences 32.8 (52.0, 39.8), one 10.3 (16.4, 9.3).
+constexpr int kStepCols = 128, kStepRows = 32, kStepRound = 128;        // (the kernel above adds up 128 rows at a time)
+template <typename T, int WAYS>
+__global__ void __launch_bounds__(WAYS * kStepCols) mamba2_step_kernel(ScanArgs a) {
+    __shared__ float sB[kStepRound], sC[kStepRound], part[WAYS][kStepCols];
     pdl_launch_dependents();
-    const int h = blockIdx.x, seq = blockIdx.y, P4 = a.P >> 2, rows = 256 / P4;
-    const int r = threadIdx.x / P4, c = threadIdx.x - r * P4, g = h / (a.heads / a.G), inner = a.heads * a.P;
+    const int h = blockIdx.x, seq = blockIdx.y, g = h / (a.heads / a.G), inner = a.heads * a.P;
+    const int cols = blockDim.x / WAYS, j = threadIdx.x / cols, c = threadIdx.x - j * cols, p = blockIdx.z * kStepCols + c;
+    const bool live = p < a.P;
     const int64_t t = a.cu_seqlens[seq];
     const T* xbc = (const T*)a.xbc + t * a.C;
     const T* proj = (const T*)a.proj + t * a.ld;
-    float4* st = reinterpret_cast<float4*>(a.state + ((int64_t)a.slots[seq] * a.heads + h) * a.N * a.P) + c;
+    float* st = a.state + (((int64_t)a.slots[seq] * a.heads + h) * a.N + j) * a.P + p;
+    const int64_t step = WAYS * (int64_t)a.P;
     const float bias = a.dt_bias[h], rate = -expf(a.a_log[h]), dskip = a.d_skip[h];
     const T* B = xbc + inner + g * a.N;
     const T* C = B + a.G * a.N;
     pdl_wait();
-    if (r < rows) {
-        // (the state's loads stand first: a warp issues in order, and would wait for the token's step size before them)
-        float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f), acc = x;
-        float da = 0.0f;
-        for (int n0 = r; n0 < a.N; n0 += 8 * rows) {
-            float4 S[8];
-            float b[8], cc[8];
+    float x = 0.0f, z = 0.0f, da = 0.0f, dtx = 0.0f, total = 0.0f;
+    for (int lo = 0; lo < a.N; lo += kStepRound) {
+        const int rows = live ? (min(kStepRound, a.N - lo) - j + WAYS - 1) / WAYS : 0;        // this thread's of the round
+        float S[kStepRows], y = 0.0f;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int n = n0 + u * rows;
-                if (n < a.N) S[u] = st[(int64_t)n * P4];
+        for (int u = 0; u < kStepRows; ++u) S[u] = u < rows ? st[u * step] : 0.0f;
+        if (lo == 0) {
+            x = live ? to_f32(xbc[h * a.P + p]) : 0.0f;
+            z = live ? to_f32(proj[h * a.P + p]) : 0.0f;
+        }
+        for (int n = threadIdx.x; n < kStepRound && lo + n < a.N; n += blockDim.x) {
+            sB[n] = to_f32(B[lo + n]);
+            sC[n] = to_f32(C[lo + n]);
+        }
+        if (lo == 0) {
+            const float dt = softplus_f(to_f32(proj[a.dt_col + h]) + bias);
+            da = expf(rate * dt);
+            dtx = dt * x;
+        }
+        __syncthreads();
+        for (int i0 = 0; i0 < rows; i0 += kStepRows) {
+            if (i0 > 0) {
+#pragma unroll
+                for (int u = 0; u < kStepRows; ++u) S[u] = i0 + u < rows ? st[(i0 + u) * step] : 0.0f;
             }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int n = n0 + u * rows;
-                if (n < a.N) {
-                    b[u] = to_f32(B[n]);
-                    cc[u] = to_f32(C[n]);
-                }
-            }
-            if (n0 == r) {
-                const T raw[4] = {xbc[h * a.P + 4 * c], xbc[h * a.P + 4 * c + 1], xbc[h * a.P + 4 * c + 2], xbc[h * a.P + 4 * c + 3]};
-                const float dt = softplus_f(to_f32(proj[a.dt_col + h]) + bias);
-                da = expf(rate * dt);
-                x = make_float4(dt * to_f32(raw[0]), dt * to_f32(raw[1]), dt * to_f32(raw[2]), dt * to_f32(raw[3]));
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int n = n0 + u * rows;
-                if (n < a.N) {
-                    S[u].x = fmaf(da, S[u].x, x.x * b[u]);
-                    S[u].y = fmaf(da, S[u].y, x.y * b[u]);
-                    S[u].z = fmaf(da, S[u].z, x.z * b[u]);
-                    S[u].w = fmaf(da, S[u].w, x.w * b[u]);
-                    acc.x = fmaf(S[u].x, cc[u], acc.x);
-                    acc.y = fmaf(S[u].y, cc[u], acc.y);
-                    acc.z = fmaf(S[u].z, cc[u], acc.z);
-                    acc.w = fmaf(S[u].w, cc[u], acc.w);
-                    st[(int64_t)n * P4] = S[u];
+            for (int u = 0; u < kStepRows; ++u) {
+                if (i0 + u < rows) {
+                    const int n = WAYS * (i0 + u) + j;
+                    S[u] = fmaf(da, S[u], dtx * sB[n]);
+                    y = fmaf(S[u], sC[n], y);
+                    st[(i0 + u) * step] = S[u];
                 }
             }
         }
-        reinterpret_cast<float4*>(part)[r * P4 + c] = acc;
+        if (WAYS > 1) {
+            part[j][c] = y;
+            __syncthreads();
+            y = (part[0][c] + part[1 % WAYS][c]) + (part[2 % WAYS][c] + part[3 % WAYS][c]);
+        }
+        total = lo == 0 ? y : total + y;
+        st += (int64_t)kStepRound * a.P;
+        __syncthreads();
     }
-    __syncthreads();
-    for (int p = threadIdx.x; p < a.P; p += 256) {
-        float y = 0.0f;
-        for (int k = 0; k < rows; ++k) y += part[k * a.P + p];
-        a.y[t * inner + h * a.P + p] = fmaf(dskip, to_f32(xbc[h * a.P + p]), y) * silu_f(to_f32(proj[h * a.P + p]));
-    }
+    if (live && j == 0) a.y[t * inner + h * a.P + p] = fmaf(dskip, x, total) * silu_f(z);
+}
+
+template <typename T>
+void launch_step(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
+    const int cols = a.P < kStepCols ? a.P : kStepCols;
+    const dim3 grid(a.heads, n_seqs, ceil_div_i(a.P, kStepCols));
+    if (a.N % 4 == 0) xs_launch(mamba2_step_kernel<T, 4>, grid, dim3(4 * cols), 0, stream, a);
+    else xs_launch(mamba2_step_kernel<T, 1>, grid, dim3(cols), 0, stream, a);
 }
 
 // Carries the state from chunk to chunk: for each (sequence, head), S = the sequence's state; for its chunks in order,
@@ -497,8 +505,8 @@ XS_API int xs_mamba2_scan(const void* xbc, const void* proj, int64_t ld, int dt_
     XS_REQUIRE(n_seqs <= 65535, "mamba2_scan: %d sequences exceed the grid limit", n_seqs);
     ScanArgs a = {xbc, proj, ld, dt_col, dt_bias, a_log, d_skip, state, cu_seqlens, slots, y, nullptr, nullptr, nullptr,
                   heads, P, N, G, heads * P + 2 * G * N, 0};
-    if (single && P % 4 == 0 && (uintptr_t)state % 16 == 0) {
-        XS_DISPATCH_DTYPE(dtype, TT, xs_launch(mamba2_step_kernel<TT>, dim3(heads, n_seqs), dim3(256), 0, stream, a));
+    if (single) {
+        XS_DISPATCH_DTYPE(dtype, TT, launch_step<TT>(a, n_seqs, stream));
         XS_LAUNCH_CHECK("mamba2_step");
         return 0;
     }
