@@ -417,6 +417,19 @@ def test_mamba2_step_is_the_scan_of_one_token(heads, P, N, G, seqs, dtype):
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+def test_mamba2_step_of_more_tokens_than_sequences_is_refused():
+    heads, P, N, G, T, seqs = 2, 8, 16, 1, 5, 3
+    inner = heads * P
+    C = inner + 2 * G * N
+    r = lambda *s: torch.randn(*s, device=DEV)                                     # noqa: E731
+    cu = torch.tensor([0, 1, 3, 5], dtype=torch.int32, device=DEV)
+    y = torch.full((T, inner), 7.0, device=DEV)
+    with pytest.raises(ops().KernelError, match="5 tokens"):
+        ops().mamba2_scan(r(T, C), r(T, inner + C + heads), inner + C, r(heads), r(heads), r(heads), r(seqs, heads, N, P), cu,
+                          torch.arange(seqs, dtype=torch.int32, device=DEV), y, heads, P, N, G, single=True)
+    assert bool((y == 7.0).all())
+
+
 @pytest.mark.parametrize("taps,C,col0,seqs", [(1, 16, 8, 2), (2, 24, 0, 1), (3, 1032, 16, 5), (4, 64, 8, 8), (5, 48, 8, 3), (4, 20, 4, 3)])
 @pytest.mark.parametrize("dtype", [torch.float32, BF])
 def test_mamba2_conv_of_single_tokens(taps, C, col0, seqs, dtype):

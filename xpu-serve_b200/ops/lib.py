@@ -1370,6 +1370,8 @@ def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: tor
     if xbc.shape[1] != heads * vdim + 2 * groups * n_state or proj.stride(1) != 1 or proj.shape[1] < dt_col + heads:
         raise KernelError(f"mamba2_scan: xbc {tuple(xbc.shape)}, proj {tuple(proj.shape)}")
     n_seqs = slots.numel()
+    if single and xbc.shape[0] != n_seqs:
+        raise KernelError(f"mamba2_scan: {xbc.shape[0]} tokens are not one for each of {n_seqs} sequences")
     if chunks is None:
         _check(load().xs_mamba2_scan(xbc.data_ptr(), proj.data_ptr(), proj.stride(0), int(dt_col), dt_bias.data_ptr(),
                                      a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), cu_seqlens.data_ptr(),
