@@ -455,6 +455,7 @@ int launch_scan(const ScanArgs& a, int units, cudaStream_t stream) {
 
 }  // namespace
 
+// Returns how many kernels ran (two where the state is moved on by a kernel of its own), or a negative code.
 XS_API int xs_mamba2_conv(const void* proj, int64_t ld, int col0, const float* taps_w, const float* bias, void* state,
                           const int32_t* seq_of_token, const int32_t* cu_seqlens, const int32_t* slots, void* out, int T,
                           int n_seqs, int C, int taps, int single, int dtype, cudaStream_t stream) {
@@ -477,7 +478,7 @@ XS_API int xs_mamba2_conv(const void* proj, int64_t ld, int col0, const float* t
 #undef XS_GO
         if (moves) {
             XS_LAUNCH_CHECK("mamba2_conv");
-            return 0;
+            return 1;
         }
     } else {
         XS_DISPATCH_DTYPE(dtype, TT,
@@ -491,7 +492,7 @@ XS_API int xs_mamba2_conv(const void* proj, int64_t ld, int col0, const float* t
                                     (const TT*)proj, ld, col0, (TT*)state, cu_seqlens, slots, C, taps));
         XS_LAUNCH_CHECK("mamba2_conv_state");
     }
-    return 0;
+    return taps > 1 ? 2 : 1;
 }
 
 // Whole sequences, one CTA per (head, sequence). single: every sequence brings exactly one token.

@@ -1349,9 +1349,10 @@ def mamba2_conv(proj: torch.Tensor, col0: int, taps_w: torch.Tensor, bias: Optio
         raise KernelError(f"mamba2_conv: state is {tuple(state.shape)}, expected [*, {taps - 1}, {C}]")
     if bias is not None:
         _need(bias, "bias", torch.float32)
-    _check(load().xs_mamba2_conv(proj.data_ptr(), proj.stride(0), int(col0), taps_w.data_ptr(), _ptr(bias), state.data_ptr(),
-                                 seq_of_token.data_ptr(), cu_seqlens.data_ptr(), slots.data_ptr(), out.data_ptr(), T,
-                                 slots.numel(), C, taps, int(single), _code(proj), _stream()), kernels=1 if taps == 1 or single else 2)
+    ran = load().xs_mamba2_conv(proj.data_ptr(), proj.stride(0), int(col0), taps_w.data_ptr(), _ptr(bias), state.data_ptr(),
+                                seq_of_token.data_ptr(), cu_seqlens.data_ptr(), slots.data_ptr(), out.data_ptr(), T, slots.numel(), C,
+                                taps, int(single), _code(proj), _stream())
+    _check(min(ran, 0), kernels=ran)
 
 
 def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor,
