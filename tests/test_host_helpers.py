@@ -120,3 +120,28 @@ def test_experts_take_the_buffers_of_their_own_route(tokens, monkeypatch):
         assert "moe_plan" in ops.ran and "moe_few_rows" not in ops.ran
         assert kept == {"moe_logits", "moe_ids", "moe_wts", "moe_place", "moe_source_padded", "moe_meta_padded", "moe_rows_in",
                         "moe_act", "moe_rows"}
+
+
+def test_a_clamped_units_product_refuses_what_its_kernel_does_not_do(monkeypatch):
+    from types import SimpleNamespace
+
+    from xpu_serve_b200.engine import runtime
+    ran = []
+    fake = SimpleNamespace(gemm_small_m_ksplit=lambda *a: 1, gemm_small_m_scratch_bytes=lambda *a: 0,
+                           gemm_small_m_clamped=lambda *a, **k: ran.append("clamped"), gemm_small_m=lambda *a, **k: ran.append("plain"))
+    monkeypatch.setattr(runtime, "ops", fake)
+    rt = runtime.Runtime.__new__(runtime.Runtime)
+    rt.sm_count, rt.gemm_scratch = 148, torch.zeros(1)
+    x, w, out, row = torch.zeros(2, 8), torch.zeros(16, 8), torch.zeros(2, 8), torch.zeros(16)
+    clamp = (7.0, 1.702, 1.0)
+    rt.few_rows_product(x, w, out, clamp=clamp)
+    assert ran == ["clamped"]
+    for extra in (dict(bias=row), dict(residual=out), dict(next_w=row), dict(next_x=x), dict(out_ssq=row), dict(conv={}), dict(argmax_into=row),
+                  dict(swiglu=True)):
+        with pytest.raises(ValueError, match="clamped"):
+            rt.few_rows_product(x, w, out, clamp=clamp, **extra)
+    with pytest.raises(ValueError, match="clamped"):
+        rt.few_rows_product(SimpleNamespace(x=x, ssq=row, width=8, eps=1e-5, shape=x.shape), w, out, clamp=clamp)
+    assert ran == ["clamped"]
+    rt.few_rows_product(x, w, out, bias=row)
+    assert ran == ["clamped", "plain"]

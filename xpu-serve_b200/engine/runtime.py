@@ -169,7 +169,11 @@ class Runtime:
         narrow; the partial sums meet in one zero-initialised scratch buffer that lives as long as
         the runtime (its tail holds the kernel's counters). `x` may be a Prenormed input; `residual`
         (the float32 stream) takes the result instead of `out`, with `next_*` / `out_ssq` as in
-        ops.gemm_small_m. `clamp` (limit, alpha, shift): the clamped unit behind a gate and up product."""
+        ops.gemm_small_m. `clamp` (limit, alpha, shift): the clamped unit behind a gate and up product, of an input that
+        carries no norm and with nothing else behind it."""
+        if clamp is not None and (hasattr(x, "ssq") or swiglu or any(v is not None for v in (bias, residual, next_w, next_x, out_ssq,
+                                                                                             conv, argmax_into))):
+            raise ValueError("the clamped unit's product takes no carried norm, bias, residual or other work behind it")
         norm = {}
         if hasattr(x, "ssq"):
             norm = dict(in_ssq=x.ssq, in_width=x.width, in_eps=x.eps)
