@@ -145,3 +145,56 @@ def test_a_clamped_units_product_refuses_what_its_kernel_does_not_do(monkeypatch
     assert ran == ["clamped"]
     rt.few_rows_product(x, w, out, bias=row)
     assert ran == ["clamped", "plain"]
+
+
+class _Places:
+    """Places as a tensor on a device has them: numbers one by one, no host array of them all."""
+
+    def __init__(self, *at):
+        self.at = at
+
+    def __len__(self):
+        return len(self.at)
+
+    def __iter__(self):
+        return (torch.tensor(p) for p in self.at)
+
+    def __array__(self, *a, **k):
+        raise TypeError("can't convert a device tensor to numpy")
+
+
+@pytest.mark.parametrize("many", [False, True])
+def test_wanted_places_may_be_whatever_gives_numbers(many):
+    from types import SimpleNamespace
+
+    import numpy as np
+
+    from xpu_serve_b200.engine.model import Model
+    from xpu_serve_b200.engine.step import StepStager
+    n = 40
+    at = list(range(1, 36)) if many else [3, 7]
+    kinds = [at, tuple(at), set(at), dict.fromkeys(at), np.asarray(at, dtype=np.uint8), torch.tensor(at), torch.tensor(at)[:, None], _Places(*at),
+             [torch.tensor(p) for p in at], [np.int64(p) for p in at], [float(p) + 0.5 for p in at], [], np.zeros(0)]
+    if many:
+        kinds.append(range(1, 36))
+    cache = SimpleNamespace(kv_groups=[], page_size=64, max_seq_tokens=64)
+    stager = StepStager("cpu")
+    ctx = stager.stage(cache, list(range(len(kinds))), [[0] * n for _ in kinds], kinds, np.zeros(len(kinds), dtype=np.int64))
+    want = [i * n + p for i, k in enumerate(kinds) for p in ([] if len(k) == 0 else at)]
+    assert ctx.want_rows.tolist() == want
+
+    class Passed(Exception):
+        pass
+
+    def begin(slots, q_lens):
+        raise Passed
+
+    model = Model.__new__(Model)
+    model.spec = SimpleNamespace(vocab=10)
+    for places in kinds:
+        with pytest.raises(Passed):                      # past the checks
+            model.step(SimpleNamespace(begin_step=begin), [0], [[1] * n], [places])
+    for bad in (-1, n):
+        for places in ([bad] + at, np.asarray([bad] + at), {bad, *at}, _Places(bad, *at), torch.tensor([bad] + at)):
+            with pytest.raises(ValueError, match="wanted place"):
+                model.step(SimpleNamespace(begin_step=begin), [0], [[1] * n], [places])

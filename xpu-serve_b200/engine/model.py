@@ -28,7 +28,7 @@ from ..ops import lib as ops
 from ..parts.block import SHARED, ResidualStream
 from ..weights.loader import load_weights
 from .runtime import Runtime, Workspace
-from .step import StepContext, StepStager
+from .step import StepContext, StepStager, places_array
 
 
 PROMPT_BUCKETS = (32, 64, 128, 256, 512)
@@ -187,9 +187,9 @@ class Model:
             raise ValueError("a step needs one token list and one list of wanted places per slot")
         token_lists = self.check_tokens(token_lists)
         for toks, places in zip(token_lists, want):
-            if len(places) >= 32:
-                at = np.asarray(places)
-                if at.ndim == 1 and at.dtype.kind == "i" and int(at.min()) >= 0 and int(at.max()) < len(toks):
+            if isinstance(places, (list, tuple, range, np.ndarray)) and len(places) >= 32:
+                at = places_array(places)
+                if int(at.min()) >= 0 and int(at.max()) < len(toks):
                     continue
             for p in places:
                 if not 0 <= int(p) < len(toks):

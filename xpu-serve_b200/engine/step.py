@@ -21,6 +21,16 @@ import numpy as np
 import torch
 
 
+def places_array(places) -> np.ndarray:
+    """Wanted places in their order as 64-bit numbers: whatever int() takes one by one (a set, a tensor on the device), lists and
+    the like at once."""
+    if isinstance(places, (list, tuple, range, np.ndarray)):
+        at = np.asarray(places, dtype=np.int64)
+        if at.ndim == 1:
+            return at
+    return np.asarray([int(p) for p in places], dtype=np.int64)
+
+
 def _round4(n: int) -> int:
     return (n + 3) & ~3
 
@@ -75,8 +85,7 @@ class StepStager:
         T = int(q_lens.sum())
         cu = np.zeros(n + 1, dtype=np.int64)
         np.cumsum(q_lens, out=cu[1:])
-        rows = [cu[i] + np.asarray(places, dtype=np.int64) for i, places in enumerate(want) if len(places)]
-        want_rows = np.concatenate(rows) if rows else np.zeros(0, dtype=np.int64)
+        want_rows = np.concatenate([np.zeros(0, dtype=np.int64)] + [cu[i] + places_array(places) for i, places in enumerate(want)])
         tables = {gi: cache.page_table(gi, slots) for gi in cache.kv_groups}
         flat = np.concatenate([np.asarray(t, dtype=np.int64) for t in token_lists]) if T else np.zeros(0, np.int64)
         seq_of = np.repeat(np.arange(n, dtype=np.int64), q_lens)
