@@ -52,6 +52,16 @@ def test_float32_product(M, N, K):
         assert torch.equal(other, out)
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two devices")
+@pytest.mark.parametrize("M", [3, 200])
+def test_float32_product_on_each_device_of_a_process(M):
+    for d in range(2):
+        with torch.cuda.device(d):
+            x, w, out = torch.randn(M, 64, device=f"cuda:{d}"), torch.randn(200, 64, device=f"cuda:{d}"), torch.empty(M, 200, device=f"cuda:{d}")
+            ops().gemm_generic(x, w, out)
+            assert gap(out, x.double() @ w.double().T) <= f32_limit(64)
+
+
 # ------------------------------------------------------------------------------------------ float32 attention
 @pytest.mark.parametrize("H,G,D,DV,planes,window,keep,plus,cap", [
     (4, 2, 64, 64, 2, 0, 0, 0, 0.0), (3, 1, 20, 36, 2, 0, 0, 0, 0.0), (2, 2, 128, 64, 2, 50, 0, 0, 0.0), (6, 2, 8, 12, 2, 33, 70, 1, 0.0),

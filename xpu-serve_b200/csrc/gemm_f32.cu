@@ -20,6 +20,8 @@
 //     N 13312 K 1024    4 rows 210 -> 13.5 (4.0 TB/s)   16 rows 212 -> 32   64 rows 221 -> 107   1,294 rows 1,569 -> 852 (41 TFLOP/s)
 //     N  1024 K 6656    4 rows 1,218 -> 14.7            16 rows 1,232 -> 20   64 rows 1,264 -> 72   1,294 rows 1,144 -> 735
 //     N 65536 K 1024    4 rows 462 -> 52 (5.2 TB/s)     16 rows 464 -> 140
+#include <atomic>
+
 #include "common.cuh"
 
 namespace {
@@ -29,6 +31,7 @@ constexpr int kStages = 3;            // of the tile kernel
 constexpr int kFewThreads = 256, kFewRows = 8;      // few rows: threads and weight rows a CTA
 constexpr int kStageK = 4 * kFewThreads;            // few rows: k of a stage, a 16-byte piece of every row a thread
 constexpr int kFewRowsMost = 64;
+constexpr int kDevices = 64;          // devices that remember their shared-memory limit (further ones set it each time)
 
 __device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // 16 bytes, of which the first `bytes` (0 to 16) are read and the rest are zeros.
@@ -244,13 +247,24 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
     }
 }
 
+// Lets a kernel of more than 48 KB of shared memory run on the current device: once a device, as the attribute is a device's.
+template <typename K>
+cudaError_t opt_in(K* kernel, size_t smem, std::atomic<bool> (&done)[kDevices]) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess || (device < kDevices && done[device].load(std::memory_order_acquire))) return e;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && device < kDevices) done[device].store(true, std::memory_order_release);
+    return e;
+}
+
 template <int MR>
 cudaError_t launch_few(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int64_t ldx, int64_t ldw,
                        int64_t ldo, cudaStream_t stream) {
     const size_t smem = (2 * (size_t)(kFewRows + MR) * kStageK + 2 * (kStageK / kChunk) * kFewRows * MR) * sizeof(float);
-    static const cudaError_t opted =
-        cudaFuncSetAttribute(gemm_f32_few_rows_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (opted != cudaSuccess) return opted;
+    static std::atomic<bool> done[kDevices];
+    const cudaError_t e = opt_in(gemm_f32_few_rows_kernel<MR>, smem, done);
+    if (e != cudaSuccess) return e;
     const int tiles = ceil_div_i(N, kFewRows), chunks = ceil_div_i(M, MR);
     const int fit = 148 * (smem <= 110 * 1024 ? 2 : 1);           // CTAs that are resident at one time
     return xs_launch(gemm_f32_few_rows_kernel<MR>, dim3(tiles < fit ? tiles : fit, chunks), dim3(kFewThreads), smem, stream, x, w, bias,
@@ -261,8 +275,9 @@ template <int BN>
 cudaError_t launch_tile(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int64_t ldx, int64_t ldw,
                         int64_t ldo, cudaStream_t stream) {
     const size_t smem = (size_t)kStages * (BM + BN) * kRow * sizeof(float);
-    static const cudaError_t opted = cudaFuncSetAttribute(gemm_f32_tile_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (opted != cudaSuccess) return opted;
+    static std::atomic<bool> done[kDevices];
+    const cudaError_t e = opt_in(gemm_f32_tile_kernel<BN>, smem, done);
+    if (e != cudaSuccess) return e;
     return xs_launch(gemm_f32_tile_kernel<BN>, dim3(ceil_div_i(N, BN), ceil_div_i(M, BM)), dim3(BN), smem, stream, x, w, bias, out, M, N, K,
                      ldx, ldw, ldo);
 }
