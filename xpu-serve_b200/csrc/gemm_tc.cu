@@ -182,7 +182,7 @@ __device__ __forceinline__ void emit16(const GemmTcParams& p, const uint32_t* r,
 // Thirty-two of them (f0 a multiple of 32), in whole 32-byte sectors where the rows allow it.
 __device__ __forceinline__ void emit32(const GemmTcParams& p, const uint32_t* r, int token, int f0) {
     if (p.vec < 2 || p.bias != nullptr || f0 + 32 > p.N || token >= p.T ||
-        (p.epilogue != EPI_STORE && (p.epilogue != EPI_SWIGLU || p.out_f32))) {
+        p.epilogue == EPI_RESIDUAL || (p.epilogue == EPI_SWIGLU && p.out_f32)) {
         emit16(p, r, token, f0);
         emit16(p, r + 16, token, f0 + 16);
         return;
@@ -202,13 +202,20 @@ __device__ __forceinline__ void emit32(const GemmTcParams& p, const uint32_t* r,
         return;
     }
     const int64_t at = (int64_t)token * p.ldo + f0;
+    const bool square = p.epilogue == EPI_RELU_SQ;
+    uint32_t v[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        const float a = fmaxf(__uint_as_float(r[j]), 0.0f);
+        v[j] = square ? __float_as_uint(a * a) : r[j];
+    }
     if (p.out_f32) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) store_32((float*)p.out + at + 8 * q, r + 8 * q);
+        for (int q = 0; q < 4; ++q) store_32((float*)p.out + at + 8 * q, v + 8 * q);
     } else {
         uint32_t o[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) o[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+        for (int j = 0; j < 16; ++j) o[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
         store_32((__nv_bfloat16*)p.out + at, o);
         store_32((__nv_bfloat16*)p.out + at + 16, o + 8);
     }
@@ -218,20 +225,27 @@ __device__ __forceinline__ void emit32(const GemmTcParams& p, const uint32_t* r,
 // columns, 32 at a time; the next 32 are on their way while these leave. `handed_back` is called when the last of them are in
 // registers. What the gated epilogue costs decides whether the next tile's products hide it: a 256 x 256 tile of K = 1024 is
 // 4.4 us of tensor-core time, and with four warps and 16-byte stores the epilogue took 15 us. Measured on B200 with the gated
-// epilogue (us, four warps -> now, L2 flushed): 8,192 tokens N 13312 K 1024 366 -> 257 (0.87 PFLOP/s; 159 storing the product as
-// it is, the vendor's product 159), 8,192 x 16384 x 2048 452 -> 383, 2,048 x 16384 x 2048 130 -> 112. (The divisions are what is
-// left of it: multiplied by an approximate reciprocal the first took 222.)
+// epilogue (us, four warps -> now, L2 flushed): 8,192 tokens N 13312 K 1024 366 -> 223 (1.00 PFLOP/s; 159 to 164 storing the
+// product as it is, the vendor's product 157), 8,192 x 16384 x 2048 452 -> 376, 2,048 x 16384 x 2048 130 -> 112.
 template <int BN, typename F>
 __device__ __forceinline__ void drain_half(const GemmTcParams& p, uint32_t acc, int half, int token, bool live, int f0, F handed_back) {
     constexpr int kParts = BN / 64;
+    static_assert(kParts % 2 == 0, "two buffers of 32 columns in turn");
     uint32_t r[2][32];
-    tmem_ask32(acc + (uint32_t)(half * (BN / 2)), r[0]);
-#pragma unroll
-    for (int c = 0; c < kParts; ++c) {
-        tmem_landed(r[c & 1]);
-        if (c + 1 < kParts) tmem_ask32(acc + (uint32_t)(half * (BN / 2) + (c + 1) * 32), r[(c + 1) & 1]);
+    const uint32_t from = acc + (uint32_t)(half * (BN / 2));
+    f0 += half * (BN / 2);
+    tmem_ask32(from, r[0]);
+    // (a loop of two parts: with all four unrolled the epilogues' code, every form of it, is there twice as often, and fetching it
+    // cost more than it saved: the first product above 257 us, 8,192 tokens N 1024 K 256 squared ReLU 25 against 17, SwiGLU 39 against 27)
+#pragma unroll 1
+    for (int c = 0; c < kParts; c += 2) {
+        tmem_landed(r[0]);
+        tmem_ask32(from + (uint32_t)((c + 1) * 32), r[1]);
+        if (live) emit32(p, r[0], token, f0 + c * 32);
+        tmem_landed(r[1]);
+        if (c + 2 < kParts) tmem_ask32(from + (uint32_t)((c + 2) * 32), r[0]);
         else handed_back();
-        if (live) emit32(p, r[c & 1], token, f0 + half * (BN / 2) + c * 32);
+        if (live) emit32(p, r[1], token, f0 + (c + 1) * 32);
     }
 }
 
