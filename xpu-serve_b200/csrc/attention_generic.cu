@@ -419,7 +419,7 @@ attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ pool
                 }
 #pragma unroll
                 for (int o = 8; o < 32; o <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, o));
-                const float corr = expf(m - m_new);                // 0 on the warp's first block (m = -inf; a block has a key)
+                const float corr = expf(m - m_new);                // 0 on the group's first block, unless no score is above the lowest number
                 float sum = 0.0f;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {

@@ -17,9 +17,18 @@
 //
 // Measured on B200 (products of the 350M shape, weights from memory, us; before: the 64 x 64 tile of gemm_generic.cu, whose time
 // does not depend on the rows):
-//     N 13312 K 1024    4 rows 210 -> 13.5 (4.0 TB/s)   16 rows 212 -> 32   64 rows 221 -> 107   1,294 rows 1,569 -> 852 (41 TFLOP/s)
+//     N 13312 K 1024    4 rows 210 -> 13.5 (4.0 TB/s)   16 rows 212 -> 32   64 rows 221 -> 76    1,294 rows 1,569 -> 852 (41 TFLOP/s)
 //     N  1024 K 6656    4 rows 1,218 -> 14.7            16 rows 1,232 -> 20   64 rows 1,264 -> 72   1,294 rows 1,144 -> 735
 //     N 65536 K 1024    4 rows 462 -> 52 (5.2 TB/s)     16 rows 464 -> 140
+// On both sides of the line between the kernels (us, L2 flushed, launch included):
+//     rows               16     64     65    128    300  1,294
+//     N 13312 K 1024     37     76    121    123    227    872     (tiles from 17 rows on)
+//     N  2048 K 1024     12     27     72     72     72    188
+//     N  1024 K 1024     10     18     72     72     72    121
+//     N  1024 K 6656     25     78    424    424    425    743
+// The line at 64 rows is right for wide outputs only. Where tiles leave most of the device idle, from 65 to some 300 rows of the
+// narrow shapes, passes of 16 rows would still be faster (K 6656: about 110 us at 96 rows); the tile there is faster than the 64 x 64
+// tile of gemm_generic.cu all the same.
 #include <atomic>
 
 #include "common.cuh"

@@ -361,7 +361,9 @@ gemm_batched_few_rows_kernel(const T* __restrict__ x, int64_t ldx, int64_t sx, c
 // The same on tensor cores (bfloat16, K a multiple of 8, rows in 16-byte pieces): 32 weight rows of one batch a CTA, whose warps
 // share K and add up in shared memory in their order. Measured on B200 (16 heads, 8 rows: N 512 K 128, and N 128 K 512): 3.8 and
 // 4.3 us; the kernel above 13.6 and 12.9, which reads 2 bytes of a weight a lane at a time behind a pass of all of x through shared
-// memory.
+// memory. Sums are the tensor core's in float32 (products of bfloat16 are exact in it) instead of fused multiply-adds, 16 k at a time
+// a warp: after the rounding to bfloat16 the errors against 64 bits are the same in all seven digits (1.67e-3, the rounding's own, at 1, 8
+// and 16 rows), and 13 of 256,000 outputs round the other way than the exact value would, 11 with the kernel above.
 template <int NT>
 __global__ void __launch_bounds__(kFewWarps * 32)
 gemm_batched_few_rows_mma_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int64_t sx, const __nv_bfloat16* __restrict__ w, int64_t ldw,
