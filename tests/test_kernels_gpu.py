@@ -559,6 +559,43 @@ def test_attention_refuses_more_splits_than_it_combines():
         run_attention(lib, Paged([100], [1], 4, 2, 64, "bfloat16"), "mma", 0.1, 0, None, 65)
 
 
+@pytest.mark.parametrize("G,Hkv,planes,window,keep", [(4, 8, 2, 0, 0), (1, 3, 2, 100, 0), (9, 1, 2, 0, 0), (16, 2, 2, -128, 0), (2, 2, 2, 64, 70),
+                                                      (4, 2, 1, 0, 0)])
+@pytest.mark.parametrize("lens", [[1, 64, 65], [512, 513, 2049, 130], [1 + 9 * i for i in range(70)]])
+def test_single_token_attention_at_the_edges_of_its_parts(G, Hkv, planes, window, keep, lens):
+    """The TMA-fed kernel: blocks dealt to its warps, keys cut into fewer parts than asked for (one up to eight blocks), more
+    (sequence, kv head) pairs than its four-warp instance takes, NaN wherever the cache holds no key. Scores of unit normals
+    over 8: weights and values rounded to bfloat16 (2^-9 each) and outputs too leave about 2^-8 of the norm."""
+    lib, n, gen = ops(), len(lens), torch.Generator(device=DEV).manual_seed(len(lens) + G)
+    pages = [-(-l // 64) for l in lens]
+    pool = torch.randn(sum(pages), planes, Hkv, 64, 64, device=DEV, generator=gen).bfloat16()
+    table = torch.full((n, max(pages) + 1), -1, dtype=torch.int32)
+    order, at = torch.randperm(sum(pages)).to(torch.int32), 0
+    for i, c in enumerate(pages):
+        table[i, :c], at = order[at:at + c], at + c
+        pool[table[i, c - 1], :, :, (lens[i] - 1) % 64 + 1:] = float("nan")
+    q = torch.randn(n, G * Hkv, 64, device=DEV, generator=gen).bfloat16()
+    cu, kv = (torch.tensor(a, dtype=torch.int32, device=DEV) for a in (range(n + 1), lens))
+    refs = []
+    for i, l in enumerate(lens):
+        k, v = (pool[table[i, :pages[i]].long().to(DEV), j].transpose(0, 1).reshape(Hkv, -1, 64)[:, :l].double() for j in (0, planes - 1))
+        key, pos = torch.arange(l, device=DEV), l - 1
+        lo = max(0, pos - window + 1) if window > 0 else pos - pos % -window if window < 0 else 0
+        sc = torch.einsum("hgd,hkd->hgk", q[i].view(Hkv, G, 64).double(), k) * 0.125
+        sc[:, :, (key < lo) & (key >= keep)] = -float("inf")
+        refs.append(torch.einsum("hgk,hkd->hgd", sc.softmax(-1), v).reshape(G * Hkv, 64))
+    ref = torch.stack(refs)
+    counters = torch.zeros(n * Hkv, dtype=torch.int32, device=DEV)
+    for splits in (1, 3, 16):
+        scratch = torch.full((max(1, lib.attention_mma_scratch_bytes(n * G * Hkv, 64, splits)),), 255, dtype=torch.uint8, device=DEV)
+        for merged in (True, False):
+            out = torch.full_like(q, float("nan"))
+            lib.attention_mma(q, pool, table.to(DEV), cu, kv, None, out, scratch, n, 1, Hkv, 64, 0.125, window, splits,
+                              counters=counters if merged else None, bounded_waits=True, keep=keep, planes=planes)
+            gap = (out.double() - ref).flatten(1).norm(dim=1) / ref.flatten(1).norm(dim=1)
+            assert gap.max() < 2 ** -7 and int(counters.abs().sum()) == 0 and lib.gemm_tc_status(DEV).item() == 0
+
+
 ATTN_TC_CASES = [
     # starts, q_lens, Hq, Hkv, window (head size 64)
     ([0], [200], 32, 8, 0),                          # the 1.2B shape's heads: 32 tokens a tile

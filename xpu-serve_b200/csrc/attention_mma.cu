@@ -26,6 +26,8 @@
 // here and served by the generic kernel. The kernels are templates in attention_mma.cuh.
 #include <cuda.h>
 
+#include <atomic>
+
 #include "attention_mma.cuh"
 #include "tc_common.cuh"
 
@@ -51,57 +53,70 @@ namespace {
 // The same decode step for head size 64 with the cache's pages brought in by the TMA unit: a page of keys (or values) of
 // one kv head is 64 x 64 contiguous bfloat16, one box of a tensor map over the whole cache, written to shared memory
 // with the 128-byte swizzle (16-byte chunk c of row r lands at chunk c ^ (r % 8), where ldmatrix then looks for it
-// without bank conflicts). A fifth warp's first lane requests pages as stages fall free; the four consumer warps wait on
-// a stage's mbarrier, multiply their 16 keys of the block and hand the stage back, so no warp waits for another inside
-// the loop, and the 1,024 predicated 16-byte copies a block cost the four warps before are two instructions. Blocks that
-// lie wholly before the sequence's newest position are requested before the wait for the kernel that writes that
+// without bank conflicts). The last warp's first lane requests pages as stages fall free. A consumer warp takes every NW-th
+// block, all 64 keys of it, on its own: it waits for that stage's mbarrier, multiplies, and hands the stage back; nothing is
+// shared between warps before the merge. A block is a chain of dependent steps (products, maximum, exponentials, products) of some
+// 0.6 us. With four warps on 16 keys each of the same block that was the time of every block, from L2 or from memory, with two
+// stages or six; now such chains run side by side, and blocks that are wholly visible skip the mask.
+// Blocks that lie wholly before the sequence's newest position are requested before the wait for the kernel that writes that
 // position. Rows past the sequence's end and pages that a window has given back come as they are (stale): their scores
-// are replaced (never multiplied) by -inf, and their value rows are zeroed in shared memory by the warp that owns them.
+// are replaced (never multiplied) by -inf, and their value rows are zeroed in shared memory by the warp that owns the block.
+// `splits` is the most parts a sequence's keys are cut into: one of fewer blocks than kPartBlocks a part is cut into fewer (a step
+// may be captured for far longer sequences than it runs with), and one of up to 2 kPartBlocks into none: a merge costs 1.5 us.
+// Measured on B200 (us, caches from memory, back to back in a graph; 32 heads over 8; before -> now): 1 sequence of 160 keys 5.7 -> 2.4,
+// of 2,112 8.4 -> 5.0; 8 of 2,112 14.0 -> 9.6 (5.3 for its bytes); 16 of 256 to 4,130 24.6 -> 18.0; 64 of 2,112 45.5 -> 42.9; 64 of
+// 16 to 200 7.1 -> 5.4.
 // Every mbarrier wait is bounded (tc_common.cuh); a CTA that gives up sets *status and writes nothing useful.
 // (KEEP_L1: the same code as a kernel of its own, so that it can carry its own preference for the split of an SM's memory
-// between shared memory and L1 cache: see g_attn_tma_carveout)
-template <int NST, bool KEEP_L1>
-__global__ void __launch_bounds__(160) attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmap_kv, const AttnParams p,
-                                                                   int* status) {
-    constexpr int D = 64, LD = D + 8, KSTEPS = D / 16, DTILES = D / 8, CHUNKS = D / 8, QROWS = 16;
+// between shared memory and L1 cache: see g_attn_tma_carveout. WIDE: more than eight heads a kv head; rows 8 to 15 of the
+// query tile are empty without it.)
+constexpr int kPartBlocks = 4;
+// Consumer warps, each with stages of its own: four while there are at most three (sequence, kv head) pairs an SM, three where there
+// are more (64 sequences of 2,112 keys, 512 pairs: four CTAs of three warps an SM are one round, 43 us; three of four two, 51 us).
+__host__ __device__ constexpr int tma_warps(bool keep_l1) { return keep_l1 ? 4 : 3; }
+
+template <int PER_WARP, bool KEEP_L1, bool WIDE>
+__global__ void __launch_bounds__(tma_warps(KEEP_L1) * 32 + 32, KEEP_L1 ? 3 : 4)
+attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmap_kv, const AttnParams p, int* status) {
+    constexpr int D = 64, KSTEPS = D / 16, DTILES = D / 8, QROWS = 16;
     constexpr int kPageBytes = BN * D * 2;                                  // 8 KB
+    // (a stage always holds the same warp's blocks: nobody else sees its phases, so nobody can take one for the next but one)
+    constexpr int NW = tma_warps(KEEP_L1), NST = NW * PER_WARP;
     extern __shared__ __align__(1024) unsigned char smem_tma[];
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_tma + 1023) & ~(uintptr_t)1023);
     unsigned char* k_sm = base;                                              // [NST][64][128 bytes], swizzled
     const bool own_v = p.planes > 1;                                         // (else the keys' rows serve as the values')
     unsigned char* v_sm = own_v ? base + NST * kPageBytes : base;
-    __nv_bfloat16* q_sm = reinterpret_cast<__nv_bfloat16*>(base + (own_v ? 2 : 1) * NST * kPageBytes);      // [16][LD]
     __shared__ __align__(8) uint64_t bar_full[NST], bar_empty[NST];
-    __shared__ float sm_m[4][QROWS], sm_l[4][QROWS];
+    __shared__ float sm_m[NW][QROWS], sm_l[NW][QROWS];
     __shared__ int pages_sm[64];
     __shared__ int abort_flag;
     __shared__ bool is_last;
 
     pdl_launch_dependents();
-    if (threadIdx.x == 128)       // the producer's lane: the tensor map on its way before the first copy asks for it
+    if (threadIdx.x == NW * 32)   // the producer's lane: the tensor map on its way before the first copy asks for it
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_kv)) : "memory");
     const int seq = blockIdx.y;
     const int kvh = blockIdx.z / p.splits, split = blockIdx.z % p.splits;
-    const int tok_begin = p.cu_seqlens[seq];
-    const int q_len = p.cu_seqlens[seq + 1] - tok_begin;
-    const int t0 = blockIdx.x * p.tokens_per_tile;
-    if (t0 >= q_len) return;
-    const int nt = min(p.tokens_per_tile, q_len - t0);
+    const int tok = p.cu_seqlens[seq];
+    if (p.cu_seqlens[seq + 1] - tok < 1) return;                              // (one token a sequence, or none)
     const int kv_len = p.kv_lens[seq];
-    const int pos0 = kv_len - q_len + t0;
-    const int hi = pos0 + nt;
-    const XsBlocks blocks = xs_blocks(pos0, hi, p.window, p.keep, BN);
-    const int bs = (int)((int64_t)blocks.count * split / p.splits);           // this CTA's share, as indices of `blocks`
-    const int be = (int)((int64_t)blocks.count * (split + 1) / p.splits);
+    const int pos = kv_len - 1;                                               // the query's position
+    const XsBlocks blocks = xs_blocks(pos, kv_len, p.window, p.keep, BN);
+    // (without counters a second kernel merges all parts: every one of them is written)
+    const int parts = p.counters == nullptr ? p.splits
+                      : blocks.count <= 2 * kPartBlocks ? 1 : min(p.splits, (blocks.count + kPartBlocks - 1) / kPartBlocks);
+    if (split >= parts) return;
+    const int bs = (int)((int64_t)blocks.count * split / parts);              // this CTA's share, as indices of `blocks`
+    const int be = (int)((int64_t)blocks.count * (split + 1) / parts);
     const int32_t* table = p.page_table + (int64_t)seq * p.P;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int G = p.G;
-    const int rows_valid = nt * G;          // <= 16
+    const int G = p.G;                                                        // <= 16
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int s = 0; s < NST; ++s) {
             mbar_init(smem_u32(&bar_full[s]), 1);
-            mbar_init(smem_u32(&bar_empty[s]), 4);             // one arrival per consumer warp
+            mbar_init(smem_u32(&bar_empty[s]), 1);             // by the warp whose block it held
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -112,12 +127,12 @@ __global__ void __launch_bounds__(160) attention_decode_tma_kernel(const __grid_
     volatile int* abort_p = &abort_flag;
     auto page_of = [&](int i) { return i - bs < 64 ? pages_sm[i - bs] : table[blocks.at(i)]; };
 
-    if (warp == 4) {
+    if (warp == NW) {
         // ------------------------------------------------------------------ producer
         if (lane == 0) {
             // the block that holds the sequence's newest position (written by the kernel before this one) and everything
             // after it wait for that kernel; earlier blocks were written by earlier steps
-            const int fresh_from = (kv_len - q_len) / BN;
+            const int fresh_from = pos / BN;
             bool waited = false;
             for (int b = bs, it = 0; b < be; ++b, ++it) {
                 const int s = it % NST;
@@ -141,35 +156,32 @@ __global__ void __launch_bounds__(160) attention_decode_tma_kernel(const __grid_
         return;
     }
 
-    // ---------------------------------------------------------------------- consumers (warps 0..3)
+    // ---------------------------------------------------------------------- consumers (the other warps)
+    const int r1 = lane >> 2, r2 = r1 + 8;                     // this lane's query rows: heads of the group
+    const int lo = xs_first_visible(pos, p.window);            // found once: may cost a division
     pdl_wait();
-    for (int c = threadIdx.x; c < QROWS * CHUNKS; c += 128) {
-        const int r = c / CHUNKS, ch = c % CHUNKS;
-        const bool ok = r < rows_valid;
-        const int ti = ok ? r / G : 0, g = ok ? r % G : 0;
-        const __nv_bfloat16* src = p.q + ((int64_t)(tok_begin + t0 + ti) * p.Hq + kvh * G + g) * D + ch * 8;
-        cp_async16(q_sm + r * LD + ch * 8, src, ok);
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    // the queries straight into the products' operand: lane (row, quarter) holds channels 2 q, 2 q + 1 of every eight
     unsigned qf[KSTEPS][4];
+    {
+        const unsigned* q1 = reinterpret_cast<const unsigned*>(p.q + ((int64_t)tok * p.Hq + kvh * G + r1) * D) + (lane & 3);
+        const unsigned* q2 = q1 + 8 * (D / 2);
 #pragma unroll
-    for (int kk = 0; kk < KSTEPS; ++kk)
-        ldmatrix_x4(qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], q_sm + (lane & 15) * LD + kk * 16 + (lane >> 4) * 8);
-
-    const int r1 = lane >> 2, r2 = r1 + 8;
-    const int pos1 = r1 < rows_valid ? pos0 + r1 / G : -1;
-    const int pos2 = r2 < rows_valid ? pos0 + r2 / G : -1;
-    const int lo1 = xs_first_visible(pos1, p.window), lo2 = xs_first_visible(pos2, p.window);     // found once: may cost a division
+        for (int kk = 0; kk < KSTEPS; ++kk) {
+            qf[kk][0] = r1 < G ? q1[kk * 8] : 0u;
+            qf[kk][2] = r1 < G ? q1[kk * 8 + 4] : 0u;
+            qf[kk][1] = WIDE && r2 < G ? q2[kk * 8] : 0u;
+            qf[kk][3] = WIDE && r2 < G ? q2[kk * 8 + 4] : 0u;
+        }
+    }
     float o[DTILES][4];
 #pragma unroll
     for (int i = 0; i < DTILES; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
     float m1 = -INFINITY, m2 = -INFINITY, l1 = 0.0f, l2 = 0.0f;
     bool bad = false;
+    const float to_log2 = p.cap_out > 0.0f ? 1.0f : p.scale_log2;
 
-    for (int i_blk = bs, it = 0; i_blk < be; ++i_blk, ++it) {
-        const int s = it % NST, b = blocks.at(i_blk);
+    for (int i_blk = bs + warp; i_blk < be; i_blk += NW) {
+        const int it = i_blk - bs, s = it % NST, b = blocks.at(i_blk);
         // (the warp decides together: its lanes poll the same barrier but may give up at different polls)
         if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_full[s]), (it / NST) & 1, abort_p))) {
             bad = true;
@@ -177,184 +189,191 @@ __global__ void __launch_bounds__(160) attention_decode_tma_kernel(const __grid_
         }
         unsigned char* ks = k_sm + s * kPageBytes;
         unsigned char* vs = v_sm + s * kPageBytes;
-        // value rows of this warp's 16 keys that hold no key of this sequence (past its end, or a page given back):
-        // zero, so that a weight of exactly 0 times stale bits stays 0
-        const int valid = page_of(i_blk) >= 0 ? min(BN, hi - b * BN) : 0;
-        if (valid < warp * 16 + 16) {
-            for (int i = lane; i < 16 * CHUNKS; i += 32) {
-                const int r = warp * 16 + i / CHUNKS;
-                if (r >= valid) *reinterpret_cast<uint4*>(vs + r * 128 + (i % CHUNKS) * 16) = make_uint4(0, 0, 0, 0);
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // before the TMA unit writes this stage again
-            __syncwarp();
-        }
-        float sc[2][4];
-        sc[0][0] = sc[0][1] = sc[0][2] = sc[0][3] = sc[1][0] = sc[1][1] = sc[1][2] = sc[1][3] = 0.0f;
+        float sc[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.0f;
 #pragma unroll
         for (int kk = 0; kk < KSTEPS; ++kk) {
-            unsigned b0, b1, b2, b3;
-            const int r = warp * 16 + (lane >> 4) * 8 + (lane & 7), ch = kk * 2 + ((lane >> 3) & 1);
-            ldmatrix_x4(b0, b1, b2, b3, ks + r * 128 + ((ch ^ (r & 7)) << 4));
-            mma_bf16(sc[0], qf[kk], b0, b1);
-            mma_bf16(sc[1], qf[kk], b2, b3);
-        }
-        const float to_log2 = p.cap_out > 0.0f ? 1.0f : p.scale_log2;
-        if (p.cap_out > 0.0f) xs_cap_scores<8>(&sc[0][0], p.cap_in, p.cap_out);
-        const int key0 = b * BN + warp * 16 + (lane & 3) * 2;
-        float mx1 = -INFINITY, mx2 = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int key = key0 + i * 8 + e;
-                const bool v1 = key <= pos1 && (key >= lo1 || key < p.keep);
-                const bool v2 = key <= pos2 && (key >= lo2 || key < p.keep);
-                sc[i][e] = v1 ? sc[i][e] * to_log2 : -INFINITY;
-                sc[i][2 + e] = v2 ? sc[i][2 + e] * to_log2 : -INFINITY;
-                mx1 = fmaxf(mx1, sc[i][e]);
-                mx2 = fmaxf(mx2, sc[i][2 + e]);
+            for (int np = 0; np < 4; ++np) {
+                unsigned b0, b1, b2, b3;
+                const int r = np * 16 + (lane >> 4) * 8 + (lane & 7), ch = kk * 2 + ((lane >> 3) & 1);
+                ldmatrix_x4(b0, b1, b2, b3, ks + r * 128 + ((ch ^ (r & 7)) << 4));
+                mma_bf16(sc[2 * np], qf[kk], b0, b1);
+                mma_bf16(sc[2 * np + 1], qf[kk], b2, b3);
             }
         }
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        mx2 = fmaxf(mx2, __shfl_xor_sync(0xffffffffu, mx2, 1));
-        mx2 = fmaxf(mx2, __shfl_xor_sync(0xffffffffu, mx2, 2));
-        const float mn1 = fmaxf(m1, mx1), mn2 = fmaxf(m2, mx2);
-        const float base1 = mn1 == -INFINITY ? 0.0f : mn1, base2 = mn2 == -INFINITY ? 0.0f : mn2;
-        const float c1 = fast_exp2(m1 - base1), c2 = fast_exp2(m2 - base2);
-        m1 = mn1;
-        m2 = mn2;
-        l1 *= c1;
-        l2 *= c2;
+        if (p.cap_out > 0.0f) xs_cap_scores<32>(&sc[0][0], p.cap_in, p.cap_out);
+        const int key0 = b * BN;
+        if (key0 + BN - 1 > pos || (key0 < lo && key0 + BN > p.keep)) {
+            // value rows that hold no key of this sequence (past its end, or a page given back): zero, so that a weight of
+            // exactly 0 times stale bits stays 0
+            const int valid = page_of(i_blk) >= 0 ? min(BN, kv_len - key0) : 0;
+            if (!own_v) __syncwarp();               // (the values are the keys' rows: every lane has read its keys)
+            for (int i = valid * 8 + lane; i < BN * 8; i += 32)
+                *reinterpret_cast<uint4*>(vs + i * 16) = make_uint4(0, 0, 0, 0);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // before the TMA unit writes this stage again
+            __syncwarp();
 #pragma unroll
-        for (int i = 0; i < DTILES; ++i) {
-            o[i][0] *= c1;
-            o[i][1] *= c1;
-            o[i][2] *= c2;
-            o[i][3] *= c2;
+            for (int i = 0; i < 8; ++i) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int key = key0 + i * 8 + (lane & 3) * 2 + e;
+                    if (key > pos || (key < lo && key >= p.keep)) sc[i][e] = sc[i][2 + e] = -INFINITY;
+                }
+            }
         }
-        unsigned pf[4];
+        // (base-2 scores: the products times to_log2, rounded once with the maximum's subtraction)
+        auto softmax = [&](int at, float& m, float& l) {
+            float mx[4];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const float p0 = fast_exp2(sc[i][0] - base1), p1 = fast_exp2(sc[i][1] - base1);
-            const float p2 = fast_exp2(sc[i][2] - base2), p3 = fast_exp2(sc[i][3] - base2);
-            l1 += p0 + p1;
-            l2 += p2 + p3;
-            pf[i * 2 + 0] = pack_bf16(p0, p1);
-            pf[i * 2 + 1] = pack_bf16(p2, p3);
-        }
+            for (int i = 0; i < 4; ++i) mx[i] = fmaxf(fmaxf(sc[i][at], sc[i][at + 1]), fmaxf(sc[i + 4][at], sc[i + 4][at + 1]));
+            float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+            const float mn = fmaxf(m, top * to_log2);
+            const float from = mn == -INFINITY ? 0.0f : mn;
+            const float c = fast_exp2(m - from);
+            m = mn;
+            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-        for (int dp = 0; dp < D / 16; ++dp) {
-            unsigned b0, b1, b2, b3;
-            const int r = warp * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), ch = dp * 2 + (lane >> 4);
-            ldmatrix_x4_trans(b0, b1, b2, b3, vs + r * 128 + ((ch ^ (r & 7)) << 4));
-            mma_bf16(o[2 * dp], pf, b0, b1);
-            mma_bf16(o[2 * dp + 1], pf, b2, b3);
+            for (int i = 0; i < 8; ++i) {
+                sc[i][at] = fast_exp2(fmaf(sc[i][at], to_log2, -from));
+                sc[i][at + 1] = fast_exp2(fmaf(sc[i][at + 1], to_log2, -from));
+                sum[i & 3] += sc[i][at] + sc[i][at + 1];
+            }
+            l = fmaf(l, c, (sum[0] + sum[1]) + (sum[2] + sum[3]));
+#pragma unroll
+            for (int i = 0; i < DTILES; ++i) {
+                o[i][at] *= c;
+                o[i][at + 1] *= c;
+            }
+        };
+        softmax(0, m1, l1);
+        if (WIDE) softmax(2, m2, l2);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            unsigned pf[4];
+            pf[0] = pack_bf16(sc[2 * kk][0], sc[2 * kk][1]);
+            pf[1] = WIDE ? pack_bf16(sc[2 * kk][2], sc[2 * kk][3]) : 0u;
+            pf[2] = pack_bf16(sc[2 * kk + 1][0], sc[2 * kk + 1][1]);
+            pf[3] = WIDE ? pack_bf16(sc[2 * kk + 1][2], sc[2 * kk + 1][3]) : 0u;
+#pragma unroll
+            for (int dp = 0; dp < D / 16; ++dp) {
+                unsigned b0, b1, b2, b3;
+                const int r = kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), ch = dp * 2 + (lane >> 4);
+                ldmatrix_x4_trans(b0, b1, b2, b3, vs + r * 128 + ((ch ^ (r & 7)) << 4));
+                mma_bf16(o[2 * dp], pf, b0, b1);
+                mma_bf16(o[2 * dp + 1], pf, b2, b3);
+            }
         }
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_empty[s])) : "memory");
     }
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    l2 += __shfl_xor_sync(0xffffffffu, l2, 1);
-    l2 += __shfl_xor_sync(0xffffffffu, l2, 2);
+    if (WIDE) {
+        l2 += __shfl_xor_sync(0xffffffffu, l2, 1);
+        l2 += __shfl_xor_sync(0xffffffffu, l2, 2);
+    }
 
-    // ---- merge the four warps through the (now idle) key stages: every consumer comes here, whatever happened before
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    // ---- merge the warps through the (now idle) key stages: every consumer comes here, whatever happened before
+    asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
     if (*abort_p || bad) {
         if (threadIdx.x == 0) atomicExch(status, 1);
-        return;                              // (the same for all 128: the flag was set before the barrier, or never)
+        return;                              // (the same for all of them: the flag was set before the barrier, or never)
     }
-    float* sm_o = reinterpret_cast<float*>(k_sm);          // [4][16][D] = 16 KB: two stages' keys
+    float* sm_o = reinterpret_cast<float*>(k_sm);          // [NW][16][D]: 4 KB a warp of the 8 that its keys had
     if ((lane & 3) == 0) {
         sm_m[warp][r1] = m1;
         sm_l[warp][r1] = l1;
-        sm_m[warp][r2] = m2;
-        sm_l[warp][r2] = l2;
+        if (WIDE) {
+            sm_m[warp][r2] = m2;
+            sm_l[warp][r2] = l2;
+        }
     }
 #pragma unroll
     for (int i = 0; i < DTILES; ++i) {
-        float* d1 = sm_o + ((warp * QROWS + r1) * D) + i * 8 + (lane & 3) * 2;
-        float* d2 = sm_o + ((warp * QROWS + r2) * D) + i * 8 + (lane & 3) * 2;
-        d1[0] = o[i][0];
-        d1[1] = o[i][1];
-        d2[0] = o[i][2];
-        d2[1] = o[i][3];
+        *reinterpret_cast<float2*>(sm_o + ((warp * QROWS + r1) * D) + i * 8 + (lane & 3) * 2) = make_float2(o[i][0], o[i][1]);
+        if (WIDE) *reinterpret_cast<float2*>(sm_o + ((warp * QROWS + r2) * D) + i * 8 + (lane & 3) * 2) = make_float2(o[i][2], o[i][3]);
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    for (int idx = threadIdx.x; idx < rows_valid * D; idx += 128) {
-        const int r = idx / D, d = idx % D;
-        float m = fmaxf(fmaxf(sm_m[0][r], sm_m[1][r]), fmaxf(sm_m[2][r], sm_m[3][r]));
-        float l = 0.0f, acc = 0.0f;
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const float f = sm_m[w][r] == -INFINITY ? 0.0f : fast_exp2(sm_m[w][r] - m);
-            l += sm_l[w][r] * f;
-            acc += sm_o[(w * QROWS + r) * D + d] * f;
+    asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
+    auto store = [&](int r, int d, float l, float m, float a0, float a1) {
+        const int h = kvh * G + r;
+        float f0 = inv_denominator(l, m, p.plus_one), f1 = f0;
+        if (p.gate != nullptr) {
+            f0 *= gate_of(p, tok, p.gate_channels ? h * D + d : h);
+            if (p.gate_channels) f1 *= gate_of(p, tok, h * D + d + 1);
+            else f1 = f0;
         }
-        const int t = tok_begin + t0 + r / G, h = kvh * G + r % G;
-        const int64_t row = (int64_t)t * p.Hq + h;
-        if (p.splits == 1) {
-            float f = inv_denominator(l, m, p.plus_one);
-            if (p.gate != nullptr) f *= gate_of(p, t, p.gate_channels ? h * D + d : h);
-            p.out[(int64_t)t * p.ld_out + h * D + d] = __float2bfloat16_rn(acc * f);
+        *reinterpret_cast<__nv_bfloat162*>(p.out + (int64_t)tok * p.ld_out + h * D + d) = __floats2bfloat162_rn(a0 * f0, a1 * f1);
+    };
+    for (int idx = threadIdx.x; idx < G * (D / 2); idx += NW * 32) {
+        const int r = idx / (D / 2), d = (idx % (D / 2)) * 2;
+        float m = sm_m[0][r];
+#pragma unroll
+        for (int w = 1; w < NW; ++w) m = fmaxf(m, sm_m[w][r]);
+        float l = 0.0f, a0 = 0.0f, a1 = 0.0f;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            const float f = sm_m[w][r] == -INFINITY ? 0.0f : fast_exp2(sm_m[w][r] - m);
+            const float2 v = *reinterpret_cast<const float2*>(sm_o + (w * QROWS + r) * D + d);
+            l += sm_l[w][r] * f;
+            a0 += v.x * f;
+            a1 += v.y * f;
+        }
+        if (parts == 1 && (p.splits == 1 || p.counters != nullptr)) {
+            store(r, d, l, m, a0, a1);
         } else {
-            p.part_o[(row * p.splits + split) * D + d] = acc;
-            if (d == 0) {
-                p.part_ml[(row * p.splits + split) * 2 + 0] = m;
-                p.part_ml[(row * p.splits + split) * 2 + 1] = l;
+            const int64_t at = ((int64_t)tok * p.Hq + kvh * G + r) * p.splits + split;
+            *reinterpret_cast<float2*>(p.part_o + at * D + d) = make_float2(a0, a1);
+            if (d == 0) *reinterpret_cast<float2*>(p.part_ml + at * 2) = make_float2(m, l);
+        }
+    }
+    if (parts == 1 || p.counters == nullptr) return;
+    // ---- the CTA of a (sequence, kv head) that stores its part last merges all of them. (One thread's fences order what the
+    // barriers on either side of them collected.)
+    asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
+    unsigned int* counter = p.counters + (int64_t)seq * p.Hkv + kvh;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        is_last = atomicAdd(counter, 1u) == (unsigned)parts - 1;
+        __threadfence();
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
+    if (!is_last) return;
+    for (int idx = threadIdx.x; idx < G * (D / 2); idx += NW * 32) {
+        const int r = idx / (D / 2), d = (idx % (D / 2)) * 2;
+        const int64_t row = (int64_t)tok * p.Hq + kvh * G + r;
+        const float* po = p.part_o + row * p.splits * D + d;
+        const float* ml = p.part_ml + row * p.splits * 2;
+        float m = -INFINITY, l = 0.0f, a0 = 0.0f, a1 = 0.0f;
+        // eight parts' sums, maxima and results asked for together: one trip to L2 for up to eight parts
+        for (int s0 = 0; s0 < parts; s0 += 8) {
+            float2 v[8], w[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                w[j] = s0 + j < parts ? __ldcg(reinterpret_cast<const float2*>(ml + 2 * (s0 + j))) : make_float2(-INFINITY, 0.0f);
+                v[j] = s0 + j < parts ? __ldcg(reinterpret_cast<const float2*>(po + (int64_t)(s0 + j) * D)) : make_float2(0.0f, 0.0f);
+            }
+            float mn = m;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) mn = fmaxf(mn, w[j].x);
+            const float from = mn == -INFINITY ? 0.0f : mn;
+            const float c = fast_exp2(m - from);
+            m = mn;
+            l *= c;
+            a0 *= c;
+            a1 *= c;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float f = fast_exp2(w[j].x - from);
+                l = fmaf(w[j].y, f, l);
+                a0 = fmaf(v[j].x, f, a0);
+                a1 = fmaf(v[j].y, f, a1);
             }
         }
-    }
-    if (p.splits == 1 || p.counters == nullptr) return;
-    // ---- the CTA of a (sequence, kv head) that stores its part last merges all of them (as attention_decode_mma_kernel)
-    __threadfence();
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    unsigned int* counter = p.counters + (int64_t)seq * p.Hkv + kvh;
-    if (threadIdx.x == 0) is_last = atomicAdd(counter, 1u) == (unsigned)p.splits - 1;
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (!is_last) return;
-    __threadfence();
-    float* w_sm = reinterpret_cast<float*>(k_sm);            // [rows][64] weights, then [rows] 1 / sum (times a head's gate)
-    float* f_sm = w_sm + QROWS * 64;
-    for (int r = warp; r < rows_valid; r += 4) {
-        const int t = tok_begin + t0 + r / G, h = kvh * G + r % G;
-        const float* ml = p.part_ml + ((int64_t)t * p.Hq + h) * p.splits * 2;
-        const float ms0 = lane < p.splits ? __ldcg(ml + 2 * lane) : -INFINITY;
-        const float ms1 = lane + 32 < p.splits ? __ldcg(ml + 2 * (lane + 32)) : -INFINITY;
-        const float ls0 = lane < p.splits ? __ldcg(ml + 2 * lane + 1) : 0.0f;
-        const float ls1 = lane + 32 < p.splits ? __ldcg(ml + 2 * (lane + 32) + 1) : 0.0f;
-        const float m = warp_max(fmaxf(ms0, ms1));
-        const float wgt0 = ms0 == -INFINITY ? 0.0f : fast_exp2(ms0 - m);
-        const float wgt1 = ms1 == -INFINITY ? 0.0f : fast_exp2(ms1 - m);
-        const float l = warp_sum(ls0 * wgt0 + ls1 * wgt1);
-        float f = inv_denominator(l, m, p.plus_one);
-        if (p.gate != nullptr && !p.gate_channels) f *= gate_of(p, t, h);
-        w_sm[r * 64 + lane] = wgt0;
-        w_sm[r * 64 + 32 + lane] = wgt1;
-        if (lane == 0) f_sm[r] = f;
-    }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    for (int idx = threadIdx.x; idx < rows_valid * (D / 2); idx += 128) {
-        const int r = idx / (D / 2), d = (idx % (D / 2)) * 2;
-        const int t = tok_begin + t0 + r / G, h = kvh * G + r % G;
-        const int64_t row = (int64_t)t * p.Hq + h;
-        const float* po = p.part_o + row * p.splits * D + d;
-        float a0 = 0.0f, a1 = 0.0f;
-#pragma unroll 8
-        for (int s = 0; s < p.splits; ++s) {
-            const float w = w_sm[r * 64 + s];
-            const float2 raw = __ldcg(reinterpret_cast<const float2*>(po + (int64_t)s * D));
-            const float2 v = w == 0.0f ? make_float2(0.0f, 0.0f) : raw;
-            a0 = fmaf(w, v.x, a0);
-            a1 = fmaf(w, v.y, a1);
-        }
-        float f0 = f_sm[r], f1 = f0;
-        if (p.gate_channels) {
-            f0 *= gate_of(p, t, h * D + d);
-            f1 *= gate_of(p, t, h * D + d + 1);
-        }
-        *reinterpret_cast<__nv_bfloat162*>(p.out + (int64_t)t * p.ld_out + h * D + d) = __floats2bfloat162_rn(a0 * f0, a1 * f1);
+        store(r, d, l, m, a0, a1);
     }
     if (threadIdx.x == 0) *counter = 0;
 }
@@ -413,42 +432,61 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_o, const
 
 // Decoding at head size 64 through the TMA-fed kernel: `map` covers the whole cache as rows of 64 elements.
 int g_attn_decode_tma = 1;        // 0: the cp.async kernel for every head size (xs_attention_mma_set_decode_tma)
-int g_attn_tma_stages = 3;
+int g_attn_tma_per_warp = 1;      // stages of a consumer warp: 1 or 2
 // Shared-memory carveout (per cent of an SM's 228 KB) that the TMA-fed kernel asks for while sequences x kv heads (its CTAs
-// before any key split) are at most three an SM: 164 KB hold three CTAs, and 64 KB stay L1 cache. Measured on B200 (1.2B shape, batch 8, whole decode step): with the
+// before any key split) are at most three an SM: 164 KB hold two CTAs, and 64 KB stay L1 cache. Measured on B200 (1.2B shape, batch 8, whole decode step): with the
 // driver's own choice for four CTAs an SM (the whole 228 KB) the step takes 0.89 ms instead of 0.75: the few-row products
 // before and after overlap this kernel on its SMs and then read their activations without an L1. Larger grids (batch 64:
 // 1.16 ms against 1.27) want the fourth CTA more. 0: always the driver's choice.
 int g_attn_tma_carveout = 72;
 
-// Shared memory of the TMA-fed kernel: stages of keys and (planes 2) values, the queries.
-size_t tma_smem(int stages, int planes) {
-    return (size_t)(planes == 1 ? 1 : 2) * stages * BN * 64 * sizeof(__nv_bfloat16) + (size_t)16 * 72 * sizeof(__nv_bfloat16) + 1024;
+// Shared memory of the TMA-fed kernel: stages of keys and (planes 2) values.
+size_t tma_smem(int stages, int planes) { return (size_t)(planes == 1 ? 1 : 2) * stages * BN * 64 * sizeof(__nv_bfloat16) + 1024; }
+
+template <int PER_WARP, bool KEEP_L1, bool WIDE>
+void tma_opt_in() {
+    static std::atomic<bool> done{false};
+    if (done.load(std::memory_order_acquire)) return;
+    auto kernel = attention_decode_tma_kernel<PER_WARP, KEEP_L1, WIDE>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem(tma_warps(KEEP_L1) * PER_WARP, 2));
+    if (KEEP_L1) cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, g_attn_tma_carveout);
+    done.store(true, std::memory_order_release);
 }
 
-template <int NST, bool KEEP_L1>
-int launch_decode_tma_as(const AttnParams& p, const CUtensorMap& map, int* status, int n_seqs, cudaStream_t stream) {
-    const size_t smem = tma_smem(NST, p.planes);
-    static bool opted = false;
-    if (!opted) {
-        cudaFuncSetAttribute(attention_decode_tma_kernel<NST, KEEP_L1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem(NST, 2));
-        if (KEEP_L1)
-            cudaFuncSetAttribute(attention_decode_tma_kernel<NST, KEEP_L1>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 g_attn_tma_carveout);
-        opted = true;
-    }
+template <int PER_WARP, bool KEEP_L1, bool WIDE>
+void launch_decode_tma_as(const AttnParams& p, const CUtensorMap& map, int* status, int n_seqs, cudaStream_t stream) {
+    tma_opt_in<PER_WARP, KEEP_L1, WIDE>();
     const dim3 grid(1, n_seqs, p.Hkv * p.splits);
-    xs_launch(attention_decode_tma_kernel<NST, KEEP_L1>, grid, dim3(160), smem, stream, map, p, status);
-    return 0;
+    xs_launch(attention_decode_tma_kernel<PER_WARP, KEEP_L1, WIDE>, grid, dim3(tma_warps(KEEP_L1) * 32 + 32),
+              tma_smem(tma_warps(KEEP_L1) * PER_WARP, p.planes), stream, map, p, status);
 }
 
 // Few CTAs before any key split (sequences x kv heads at most three an SM): the instance that keeps an L1.
 bool tma_keeps_l1(int64_t tiles) { return g_attn_tma_carveout > 0 && tiles <= (int64_t)3 * sm_count(); }
 
-template <int NST>
-int launch_decode_tma(const AttnParams& p, const CUtensorMap& map, int* status, int n_seqs, cudaStream_t stream) {
-    if (tma_keeps_l1((int64_t)n_seqs * p.Hkv)) return launch_decode_tma_as<NST, true>(p, map, status, n_seqs, stream);
-    return launch_decode_tma_as<NST, false>(p, map, status, n_seqs, stream);
+template <int PER_WARP>
+void launch_decode_tma(const AttnParams& p, const CUtensorMap& map, int* status, int n_seqs, cudaStream_t stream) {
+    const bool keep = tma_keeps_l1((int64_t)n_seqs * p.Hkv);
+    if (p.G > 8) keep ? launch_decode_tma_as<PER_WARP, true, true>(p, map, status, n_seqs, stream) : launch_decode_tma_as<PER_WARP, false, true>(p, map, status, n_seqs, stream);
+    else keep ? launch_decode_tma_as<PER_WARP, true, false>(p, map, status, n_seqs, stream) : launch_decode_tma_as<PER_WARP, false, false>(p, map, status, n_seqs, stream);
+}
+
+// CTAs of it an SM.
+template <int PER_WARP, bool KEEP_L1>
+int tma_per_sm(int planes) {
+    static int cached[2] = {};
+    int& per = cached[planes > 1 ? 1 : 0];
+    if (per == 0) {
+        const size_t smem = tma_smem(tma_warps(KEEP_L1) * PER_WARP, planes);
+        int got = 0;
+        tma_opt_in<PER_WARP, KEEP_L1, false>();
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&got, attention_decode_tma_kernel<PER_WARP, KEEP_L1, false>, tma_warps(KEEP_L1) * 32 + 32, smem);
+        // (the occupancy query may not know of the carveout: 164 KB hold two CTAs of four stages)
+        const int room = (int)((size_t)g_attn_tma_carveout * 228 * 1024 / 100 / (smem + 1024));
+        if (KEEP_L1 && got > room) got = room;
+        per = got > 0 ? got : 1;
+    }
+    return per;
 }
 
 }  // namespace
@@ -478,34 +516,9 @@ XS_API int xs_attention_mma_set_decode_stages(int n) {
 XS_API int xs_attention_mma_decode_slots(int D, int DV, int planes, int64_t tiles) {
     if (D != DV) return pair_decode_slots(D, DV, tiles);
     if (D == 64 && g_attn_decode_tma && encode_fn() != nullptr) {       // the TMA-fed kernel: its own occupancy
-        static int per_sm[8][2][2] = {};
-        const int n = g_attn_tma_stages, k = tma_keeps_l1(tiles) ? 1 : 0, own = planes > 1 ? 1 : 0;
-        if (per_sm[n][k][own] == 0) {
-            const size_t smem = tma_smem(n, planes);
-            int got = 0;
-#define XS_TMA_OCC(NST, KEEP)                                                                                                \
-    do {                                                                                                                     \
-        cudaFuncSetAttribute(attention_decode_tma_kernel<NST, KEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem(NST, 2)); \
-        if (KEEP)                                                                                                            \
-            cudaFuncSetAttribute(attention_decode_tma_kernel<NST, KEEP>, cudaFuncAttributePreferredSharedMemoryCarveout,     \
-                                 g_attn_tma_carveout);                                                                       \
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&got, attention_decode_tma_kernel<NST, KEEP>, 160, smem);              \
-    } while (0)
-#define XS_TMA_OCC2(NST) if (k) XS_TMA_OCC(NST, true); else XS_TMA_OCC(NST, false)
-            switch (n) {
-                case 2: XS_TMA_OCC2(2); break;
-                case 3: XS_TMA_OCC2(3); break;
-                case 5: XS_TMA_OCC2(5); break;
-                case 6: XS_TMA_OCC2(6); break;
-                default: XS_TMA_OCC2(4); break;
-            }
-#undef XS_TMA_OCC2
-#undef XS_TMA_OCC
-            // (the occupancy query may not know of the carveout: 164 KB hold three CTAs of three stages)
-            if (k && got > (int)((size_t)g_attn_tma_carveout * 228 * 1024 / 100 / (smem + 1024))) got = (int)((size_t)g_attn_tma_carveout * 228 * 1024 / 100 / (smem + 1024));
-            per_sm[n][k][own] = got > 0 ? got : 1;
-        }
-        return sm_count() * per_sm[n][k][own];
+        const bool keep = tma_keeps_l1(tiles);
+        if (g_attn_tma_per_warp == 2) return sm_count() * (keep ? tma_per_sm<2, true>(planes) : tma_per_sm<2, false>(planes));
+        return sm_count() * (keep ? tma_per_sm<1, true>(planes) : tma_per_sm<1, false>(planes));
     }
     switch (D) {
         case 16: return decode_slots<16, 16>(tiles);
@@ -531,7 +544,7 @@ XS_API int xs_attention_mma_supports(int D, int DV, int page_size, int G) {
 
 XS_API void xs_attention_mma_set_decode_tma(int on, int stages) {
     g_attn_decode_tma = on ? 1 : 0;
-    if (stages >= 2 && stages <= 6) g_attn_tma_stages = stages;
+    if (stages >= 2 && stages <= 6) g_attn_tma_per_warp = stages <= 4 ? 1 : 2;
 }
 XS_API void xs_attention_mma_set_tma_carveout(int percent) { g_attn_tma_carveout = percent; }
 
@@ -597,13 +610,8 @@ XS_API int xs_attention_mma_merged(const void* q, const void* pool, const int32_
         encode_fn() != nullptr) {
         alignas(64) CUtensorMap map;
         XS_REQUIRE(make_map(&map, pool, pool_pages * planes * Hkv * BN, D, D, BN), "attention: the cache's tensor map could not be made");
-        switch (g_attn_tma_stages) {
-            case 2: launch_decode_tma<2>(p, map, status, n_seqs, stream); break;
-            case 3: launch_decode_tma<3>(p, map, status, n_seqs, stream); break;
-            case 5: launch_decode_tma<5>(p, map, status, n_seqs, stream); break;
-            case 6: launch_decode_tma<6>(p, map, status, n_seqs, stream); break;
-            default: launch_decode_tma<4>(p, map, status, n_seqs, stream); break;
-        }
+        if (g_attn_tma_per_warp == 2) launch_decode_tma<2>(p, map, status, n_seqs, stream);
+        else launch_decode_tma<1>(p, map, status, n_seqs, stream);
     } else
     switch (D) {
         case 16: launch<16, 16>(p, max_tiles, n_seqs, stream); break;
