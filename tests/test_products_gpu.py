@@ -356,6 +356,31 @@ def test_experts_rows_do_not_depend_on_the_step():
         assert torch.equal(one, whole[2 * t:2 * t + 2])
 
 
+@pytest.mark.parametrize("T,top,E,N,K", [(1, 1, 3, 16, 8), (1, 4, 16, 2048, 520), (2, 2, 9, 2032, 64), (8, 4, 16, 200, 1000), (8, 2, 40, 1040, 2048),
+                                         (5, 5, 150, 144, 2816), (9, 2, 4, 272, 72), (16, 4, 16, 256, 2048), (16, 2, 5, 130, 2056), (8, 1, 2, 48, 4096),
+                                         (3, 2, 4, 40, 9400)])
+def test_streamed_experts_at_their_lines(T, top, E, N, K):
+    """Four and eight warps a CTA, one and two groups of eight rows, K past whole stages, rows of x that leave room for two CTAs
+    an SM, for one or for none. One infinite input: its row alone is affected, and stays infinite where the sign is certain."""
+    x, w = torch.randn(T, K, device=DEV).to(BF), (torch.randn(E, N, K, device=DEV) / math.sqrt(K)).to(BF)
+    ids = torch.stack([torch.randperm(E, device=DEV)[:top] for _ in range(T)]).to(torch.int32)
+    ids[0, 0] = -1
+    ids = ids.reshape(-1)
+    out = torch.full((T * top, N), 7.0, device=DEV, dtype=BF)
+    ops().moe_few_rows(x, top, w, out, ids, T, glu=False)
+    ref = torch.einsum("rnk,rk->rn", w[ids.long().clamp(min=0)].double(), x.double().repeat_interleave(top, 0))
+    met = ids >= 0
+    assert gap(out[met], ref[met]) <= 2.0 ** -8 if bool(met.any()) else True
+    assert bool((out[~met] == 7.0).all())
+    x[T - 1, K - 1] = math.inf
+    again = torch.full_like(out, 7.0)
+    ops().moe_few_rows(x, top, w, again, ids, T, glu=False)
+    assert torch.equal(again[:(T - 1) * top], out[:(T - 1) * top])
+    last = met[(T - 1) * top:]
+    sign = w[ids[(T - 1) * top:].long().clamp(min=0), :, K - 1].sign()
+    assert bool((again[(T - 1) * top:] == sign * math.inf)[last].logical_or(sign[last] == 0).all())
+
+
 # ------------------------------------------------------------------------- kernels of the recurrent and latent layers
 @pytest.mark.parametrize("B,M,N,K", [(1, 1, 1, 8), (16, 8, 512, 128), (3, 9, 33, 520), (2, 16, 31, 1032), (4, 5, 100, 24)])
 def test_batched_product_of_few_rows(B, M, N, K):
