@@ -328,6 +328,35 @@ def test_a_token_of_nan_leaves_the_others_alone():
         ops().moe_few_rows(x, top, w, out, ids, 7, glu=False)
 
 
+@pytest.mark.parametrize("T,clamped", [(150, False), (300, False), (300, True)])
+@pytest.mark.parametrize("out_dtype", [BF, torch.float32])
+def test_gated_epilogue_over_all_gates(T, clamped, out_dtype):
+    """Gates from the most negative to the largest, where e^-g leaves the normal numbers and where the division takes over; NaN stays
+    NaN. Every result is its own quotient: half a unit in the last place of the stored type, and e^-g's few units of float32."""
+    g = torch.cat([torch.linspace(-100, 20, T - 12), torch.tensor([-3.3e38, -1e30, -200.0, -88.5, -87.0, -86.9, 0.0, -0.0, 1e-38, 100.0, 1e30, 1e38])])
+    x = torch.zeros(T, 64, device=DEV, dtype=BF)
+    x[:, 0], x[:, 1] = g.to(DEV), torch.linspace(-3, 3, T, device=DEV)
+    x[5, 0] = math.nan
+    w = torch.zeros(8, 2, 8, 64, device=DEV, dtype=BF)
+    w[:, 0, :, 0] = w[:, 1, :, 1] = 1.0
+    out = torch.zeros(T, 64, device=DEV, dtype=out_dtype)
+    g, u = x[:, :1].double(), x[:, 1:2].double()
+    if clamped:
+        ops().gemm_tc_clamped(x, w.view(128, 64), out, 7.0, 1.702, 1.0)
+        g, u, a = g.clamp(max=7.0), u.clamp(-7.0, 7.0) + 1.0, 1.702
+    else:
+        ops().gemm_tc(x, w.view(128, 64), out, epilogue=ops().EPI_SWIGLU)
+        a = 1.0
+    ref = (g * torch.sigmoid(a * g) * u).expand(T, 64)
+    keep = torch.arange(T, device=DEV) != 5
+    assert bool(out[5].isnan().all()) or clamped
+    if not clamped:
+        # (e^-g beyond the largest number: the quotient is 0; 1e-36 covers it)
+        assert bool(((out.double() - ref).abs()[keep] <= (2.0 ** -8 if out_dtype == BF else 2.0 ** -18) * ref.abs()[keep] + 1e-36).all())
+    else:
+        assert bool(((out.double() - ref).abs()[keep] <= 2.0 ** -8 * ref.abs()[keep] + 1e-35).all())
+
+
 @pytest.mark.parametrize("M,F,K", [(1, 8, 8), (3, 24, 264), (8, 1024, 2048), (8, 16, 8192), (9, 40, 1032), (16, 1024, 2048)])
 @pytest.mark.parametrize("slices", [1, 4])
 def test_clamped_unit_of_few_rows(M, F, K, slices):

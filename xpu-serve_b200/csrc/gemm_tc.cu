@@ -67,6 +67,43 @@ __device__ __forceinline__ float gated_unit(const GemmTcParams& p, float g, floa
     return g / (1.0f + __expf(-g)) * u;
 }
 
+// n results of the gated unit: a[j] from gate v[at(j)] and up v[at(j) + 8].
+// A division that compiles to a branch per result (its rare ranges) leaves the results one after another: 16 of them took 1,800
+// cycles of two warps a scheduler, more than the products of a tile of K = 1024. Where all of a thread's gates are ordinary (-87 to the largest
+// finite number, so that 1 + e^-g and its reciprocal are normal numbers) the quotient is formed without one: the hardware's
+// reciprocal r of d, q = g r, and one correction by the exact residual, q + (g - q d) r (Newton's step for a quotient as in Markstein,
+// IBM J. Res. Dev. 34, 1990), which leaves half a unit in the last place and 2^-22 of it. Results next to a rounding boundary aside it is
+// the division's; anything else takes the division.
+__device__ __forceinline__ float as_f32(float v) { return v; }
+__device__ __forceinline__ float as_f32(uint32_t v) { return __uint_as_float(v); }
+template <int N, typename V, typename At>
+__device__ __forceinline__ void gated_units(const GemmTcParams& p, const V* v, float* a, At at) {
+    if (p.glu_act == 0) {
+        const bool clamped = p.glu_limit > 0.0f;
+        const float alpha = clamped ? p.glu_alpha : 1.0f;
+        bool plain = true;
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            float g = as_f32(v[at(j)]), u = as_f32(v[at(j) + 8]);
+            plain = plain && g <= 3.0e38f;
+            if (clamped) {
+                g = fminf(g, p.glu_limit);
+                u = fminf(fmaxf(u, -p.glu_limit), p.glu_limit) + p.glu_shift;
+            }
+            const float x = alpha * g;
+            plain = plain && x >= -87.0f && g >= -3.0e38f;
+            const float d = 1.0f + __expf(-x);
+            float r;
+            asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+            const float q = g * r;
+            a[j] = fmaf(fmaf(-q, d, g), r, q) * u;
+        }
+        if (plain) return;
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) a[j] = gated_unit(p, as_f32(v[at(j)]), as_f32(v[at(j) + 8]));
+}
+
 // Instruction descriptor of this file's single-CTA products: M = 128, N = n.
 __host__ __device__ constexpr uint32_t instr_desc(int n) { return instr_desc_mn(BM, n); }
 
@@ -124,8 +161,7 @@ __device__ __forceinline__ void emit16(const GemmTcParams& p, const uint32_t* r,
     }
     if (p.epilogue == EPI_SWIGLU) {   // rows f0..f0+7 are gates, f0+8..f0+15 their up rows; N is a multiple of 16
         float a[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = gated_unit(p, v[j], v[j + 8]);
+        gated_units<8>(p, v, a, [](int j) { return j; });
         const int64_t at = (int64_t)token * p.ldo + (f0 >> 1);
         if (p.out_f32) {
             float* o = (float*)p.out + at;
@@ -189,11 +225,7 @@ __device__ __forceinline__ void emit32(const GemmTcParams& p, const uint32_t* r,
     }
     if (p.epilogue == EPI_SWIGLU) {
         float a[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int g = (j & 7) + (j >> 3) * 16;
-            a[j] = gated_unit(p, __uint_as_float(r[g]), __uint_as_float(r[g + 8]));
-        }
+        gated_units<16>(p, r, a, [](int j) { return (j & 7) + (j >> 3) * 16; });
         const int64_t at = (int64_t)token * p.ldo + (f0 >> 1);
         uint32_t o[8];
 #pragma unroll
@@ -225,8 +257,10 @@ __device__ __forceinline__ void emit32(const GemmTcParams& p, const uint32_t* r,
 // columns, 32 at a time; the next 32 are on their way while these leave. `handed_back` is called when the last of them are in
 // registers. What the gated epilogue costs decides whether the next tile's products hide it: a 256 x 256 tile of K = 1024 is
 // 4.4 us of tensor-core time, and with four warps and 16-byte stores the epilogue took 15 us. Measured on B200 with the gated
-// epilogue (us, four warps -> now, L2 flushed): 8,192 tokens N 13312 K 1024 366 -> 223 (1.00 PFLOP/s; 159 to 164 storing the
-// product as it is, the vendor's product 157), 8,192 x 16384 x 2048 452 -> 376, 2,048 x 16384 x 2048 130 -> 112.
+// epilogue (us, L2 flushed; four warps -> eight warps and 32-byte stores -> without the branch of each division, see gated_units):
+// 8,192 tokens N 13312 K 1024 366 -> 225 -> 182 (1.23 PFLOP/s; 165 storing the product as it is, the vendor's product 157), 2,048
+// tokens 71 -> 58, 512 tokens 34 -> 28; 8,192 x 1024 x 256 32 -> 21; 8,192 x 16384 x 2048 452 -> 380 (level since: the tensor
+// core's), 512 x 16384 x 2048 44 -> 40.
 template <int BN, typename F>
 __device__ __forceinline__ void drain_half(const GemmTcParams& p, uint32_t acc, int half, int token, bool live, int f0, F handed_back) {
     constexpr int kParts = BN / 64;
