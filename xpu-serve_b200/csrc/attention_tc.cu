@@ -4,10 +4,10 @@
 // group, G = heads / kv_heads) and walks the cache in blocks of 128 keys (two pages). Per block:
 //
 //   warp 0   TMA producer: the block's K and V pages (64 x 64 elements each, 128-byte swizzle) into a
-//            ring of three stages. Pages past the sequence's end, pages a window has given back, and the
+//            ring of four stages (each group works on one and waits for the next). Pages past the sequence's end, pages a window has given back, and the
 //            rows of the last page past the sequence's length are zeroed in shared memory (V only: a
 //            masked score becomes a weight of exactly 0, and 0 times stale bits must stay 0).
-//   warp 1 and warp 10: one thread each issues S = Q K^T and O += P V:
+//   warp 1 and warp 10: one lane of each issues S = Q K^T and O += P V:
 //   warp 1   one thread issues S = Q K^T (tcgen05.mma, M 128, N 128, K 16 x D / 16, Q and K K-major) into
 //            one of two S buffers in tensor memory, and O += P V (M 128, N D, K 16 x 8, P K-major from
 //            shared memory, V MN-major: the pages' own layout) into the output, which stays in tensor memory.
@@ -17,8 +17,13 @@
 //            rescale their halves of its output in tensor memory (tcgen05.ld, multiply, tcgen05.st) before
 //            they hand the block's P over; the output is read once, at the end.
 //
-// S of block j + 1 is issued before P V of block j, so the tensor pipe works while the softmax of block j
-// runs. Every mbarrier wait is bounded (see tc_common.cuh); a CTA that gives up frees its tensor memory and
+// A group's next S is issued as soon as it has read its scores, and runs under its softmax. A group's weights wait for its previous
+// P V: it reads the memory they are written to. Measured on B200 (us; 16 heads over 8): 8,192 tokens 314 -> 273, behind 8,192 more 782
+// -> 661 (624 TFLOP/s), 32 heads over 8, four times 2,048 252 -> 232: with three stages of pages the next pages' way from
+// memory stood in front of every second S (752 us), and the scores' buffer went back only with the weights. The exponential unit is
+// then 54 % busy: its 128 results a thread take 2,000 of a group's 3,700 cycles a block. Tried instead: P in tensor memory 733, three groups of
+// 64-key blocks 788, two threads a row 1,153, every eighth exponential as a polynomial on the FMA units 809 (registers).
+// Every mbarrier wait is bounded (see tc_common.cuh); a CTA that gives up frees its tensor memory and
 // sets *status. A window may keep the sequence's first positions visible: their blocks are walked before the window's; a cache
 // with one plane holds keys that are the values too. Head size 64, groups that divide 128, one key split; other cases take the mma.sync kernel.
 // The reference's counterpart is its XMX flash kernel for prefill (src/backend/sycl/sycl_flash_attention.cpp:1-15).
@@ -33,7 +38,7 @@ constexpr int TM = 128;           // query rows a CTA
 constexpr int TN = 128;           // keys a block
 constexpr int PAGE = 64;          // keys a page
 constexpr int kAttnThreads = 352;   // TMA warp, S issuer warp, eight softmax warps, P V issuer warp
-constexpr int KV_STAGES = 3;
+constexpr int KV_STAGES = 4;
 
 struct AttnTcParams {
     const __nv_bfloat16* q;          // [T, Hq, D]
@@ -78,22 +83,8 @@ __device__ __forceinline__ void tmem_ld32_nowait(uint32_t addr, uint32_t* r) {
         : "r"(addr));
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld16w(uint32_t addr, uint32_t* r) {     // 16 columns, waited for
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(addr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_st16w(uint32_t addr, const uint32_t* r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 :: "r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-                 : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-// tcgen05.st of 32 columns of this thread's lane, and the wait for it
-__device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t* r) {
+// tcgen05.st of 32 columns of this thread's lane; tmem_st_wait() waits for all that were asked for
+__device__ __forceinline__ void tmem_st32_nowait(uint32_t addr, const uint32_t* r) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
         "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
@@ -102,7 +93,14 @@ __device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t* r) {
            "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
            "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// True in one lane of the (whole) warp, chosen so that the compiler knows that one lane is active behind it and keeps the products'
+// operands in uniform registers.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
 }
 // Descriptor of an MN-major operand with the 128-byte swizzle: 64 elements of N contiguous (128 bytes), rows of
 // K 128 bytes apart, groups of 8 rows of K 1024 bytes apart (stride byte offset). One 64-wide chunk of N only,
@@ -254,44 +252,65 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const AttnTcPar
         // ------------------------------------------------------------------ issuer of S = Q K^T
         // (two issuing threads, this one and warp 10's: one thread's descriptor arithmetic and waits for both
         // products of a block took longer than the block's softmax)
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = instr_desc_mn(TM, TN);
-            const uint64_t dq = smem_desc_sw128(smem_u32(q_sm));
-            const uint64_t dk0 = smem_desc_sw128(smem_u32(kv_sm));
-            for (int j = 0; j < nb && !*abort_p; ++j) {
-                const int s = j % KV_STAGES, buf = j & 1;
-                if (!mbar_wait(smem_u32(&bar_kv_full[s]), (j / KV_STAGES) & 1, abort_p)) break;
-                if (j >= 2 && !mbar_wait(smem_u32(&bar_s_empty[buf]), ((j >> 1) & 1) ^ 1, abort_p)) break;
-                tcgen05_fence_after();
-                const uint64_t dk = dk0 + (uint64_t)(s * (kStageBytes >> 4));      // start addresses count 16 bytes
+        // The whole warp walks the blocks, so that addresses and descriptors stay in uniform registers, and one lane issues.
+        const bool lead = elect_one();
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+        constexpr uint32_t idesc_s = instr_desc_mn(TM, TN);
+        const uint64_t dq = smem_desc_sw128(smem_u32(q_sm));
+        const uint64_t dk0 = smem_desc_sw128(smem_u32(kv_sm));
+        int s = 0, turn = 0;                                   // stage, and how often the ring has gone round
+        bool ok = true;
+        for (int j0 = 0, n = 0; j0 < nb && ok; j0 += 2, ++n) {          // the n-th block of either group
 #pragma unroll
-                for (int k = 0; k < D / 16; ++k)
-                    umma_bf16(tmem_base + (uint32_t)(buf * TN), dq + (uint64_t)(k * 2), dk + (uint64_t)(k * 2), idesc_s, k > 0 ? 1u : 0u);
-                tcgen05_commit(smem_u32(&bar_s_full[buf]));
+            for (int buf = 0; buf < 2; ++buf) {
+                if (j0 + buf >= nb || !ok) break;
+                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_kv_full[s]), turn & 1, abort_p) &&
+                                                 (n == 0 || mbar_wait(smem_u32(&bar_s_empty[buf]), (n - 1) & 1, abort_p)));
+                if (!ok) break;
+                tcgen05_fence_after();
+                if (lead) {
+                    const uint64_t dk = dk0 + (uint64_t)(s * (kStageBytes >> 4));      // start addresses count 16 bytes
+#pragma unroll
+                    for (int k = 0; k < D / 16; ++k)
+                        umma_bf16(tm + (uint32_t)(buf * TN), dq + (uint64_t)(k * 2), dk + (uint64_t)(k * 2), idesc_s, k > 0 ? 1u : 0u);
+                    tcgen05_commit(smem_u32(&bar_s_full[buf]));
+                }
+                __syncwarp();
+                if (++s == KV_STAGES) s = 0, ++turn;
             }
         }
     } else if (warp == 10) {
         // ------------------------------------------------------------------ issuer of O += P V
-        if (lane == 0) {
-            constexpr uint32_t idesc_o = instr_desc_mn(TM, D, true);
-            const uint64_t dp0 = smem_desc_sw128(smem_u32(p_sm));
-            const uint64_t dv0 = smem_desc_sw128_mn(smem_u32(kv_sm + (own_v ? 2 * kPageBytes : 0)));
-            for (int j = 0; j < nb && !*abort_p; ++j) {
-                const int s = j % KV_STAGES, buf = j & 1;
-                if (!mbar_wait(smem_u32(&bar_kv_full[s]), (j / KV_STAGES) & 1, abort_p)) break;
-                if (!mbar_wait(smem_u32(&bar_p_full[buf]), (j >> 1) & 1, abort_p)) break;
-                tcgen05_fence_after();
-                const uint64_t dp = dp0 + (uint64_t)(buf * (kPBytes >> 4));
-                const uint64_t dv = dv0 + (uint64_t)(s * (kStageBytes >> 4));
+        const bool lead = elect_one();
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+        constexpr uint32_t idesc_o = instr_desc_mn(TM, D, true);
+        const uint64_t dp0 = smem_desc_sw128(smem_u32(p_sm));
+        const uint64_t dv0 = smem_desc_sw128_mn(smem_u32(kv_sm + (own_v ? 2 * kPageBytes : 0)));
+        int s = 0, turn = 0;
+        bool ok = true;
+        for (int j0 = 0, n = 0; j0 < nb && ok; j0 += 2, ++n) {
 #pragma unroll
-                for (int k = 0; k < TN / 16; ++k) {
-                    // P: K-major, 16 keys = 32 bytes along a row, the second 64 keys in the second half tile;
-                    // V: MN-major, 16 keys = 16 rows of 128 bytes
-                    umma_bf16(tmem_base + kColO + (uint32_t)(buf * D), dp + (uint64_t)((k >> 2) * ((TM * 128) >> 4) + (k & 3) * 2),
-                              dv + (uint64_t)(k * ((16 * 128) >> 4)), idesc_o, (j >= 2 || k > 0) ? 1u : 0u);   // adds up over the group's blocks
+            for (int buf = 0; buf < 2; ++buf) {
+                if (j0 + buf >= nb || !ok) break;
+                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_kv_full[s]), turn & 1, abort_p) &&
+                                                 mbar_wait(smem_u32(&bar_p_full[buf]), n & 1, abort_p));
+                if (!ok) break;
+                tcgen05_fence_after();
+                if (lead) {
+                    const uint64_t dp = dp0 + (uint64_t)(buf * (kPBytes >> 4));
+                    const uint64_t dv = dv0 + (uint64_t)(s * (kStageBytes >> 4));
+#pragma unroll
+                    for (int k = 0; k < TN / 16; ++k) {
+                        // P: K-major, 16 keys = 32 bytes along a row, the second 64 keys in the second half tile;
+                        // V: MN-major, 16 keys = 16 rows of 128 bytes
+                        umma_bf16(tm + kColO + (uint32_t)(buf * D), dp + (uint64_t)((k >> 2) * ((TM * 128) >> 4) + (k & 3) * 2),
+                                  dv + (uint64_t)(k * ((16 * 128) >> 4)), idesc_o, (n > 0 || k > 0) ? 1u : 0u);   // adds up over the group's blocks
+                    }
+                    tcgen05_commit(smem_u32(&bar_o_done[buf]));
+                    tcgen05_commit(smem_u32(&bar_kv_empty[s]));
                 }
-                tcgen05_commit(smem_u32(&bar_o_done[buf]));
-                tcgen05_commit(smem_u32(&bar_kv_empty[s]));
+                __syncwarp();
+                if (++s == KV_STAGES) s = 0, ++turn;
             }
         }
     } else {
@@ -322,6 +341,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const AttnTcPar
 #pragma unroll
             for (int c = 0; c < TN; c += 32) tmem_ld32_nowait(lane_base + s_col + (uint32_t)c, raw + c);
             tmem_ld_wait();
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cta(smem_u32(&bar_s_empty[grp]));       // the group's next scores may come
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
             if constexpr (CAP) {
                 // (columns that hold no key may hold anything here: they are replaced below)
@@ -354,21 +376,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const AttnTcPar
             const float mb = m_new == -INFINITY ? 0.0f : m_new;
             const float alpha = ex2(m - mb);                      // 0 while nothing was seen
             m = m_new;
-            if (done >= 1 && __any_sync(0xffffffffu, alpha != 1.0f)) {
-                // The group's output so far lives in tensor memory, relative to the old maximum: rescale this row
-                // before this block's P V adds to it. That product waits for this warp's arrival below, the one
-                // before it is waited for here. The maximum of most later blocks does not move.
-                if (!mbar_wait(smem_u32(&bar_o_done[grp]), (done - 1) & 1, abort_p)) { bad = true; break; }
-                tcgen05_fence_after();
-#pragma unroll 1
-                for (int c = 0; c < D; c += 16) {                  // 16 columns at a time: the scores stay in registers
-                    uint32_t acc[16];
-                    tmem_ld16w(lane_base + o_col + (uint32_t)c, acc);
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
-                    tmem_st16w(lane_base + o_col + (uint32_t)c, acc);
-                }
-            }
+            // the group's P V before this block's has read P and is in O (it ran under this block's maximum)
+            if (done >= 1 && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_o_done[grp]), (done - 1) & 1, abort_p))) { bad = true; break; }
+            tcgen05_fence_after();
             float add4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             uint8_t* p_row = p_sm + grp * kPBytes + r * 128;
 #pragma unroll
@@ -383,13 +393,23 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const AttnTcPar
                     make_uint4(pack_bf16(w[0], w[1]), pack_bf16(w[2], w[3]), pack_bf16(w[4], w[5]), pack_bf16(w[6], w[7]));
             }
             l = l * alpha + ((add4[0] + add4[1]) + (add4[2] + add4[3]));
+            if (done >= 1 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+                // The group's output so far lives in tensor memory, relative to the old maximum: rescale this row before this block's
+                // P V adds to it. Behind the weights the scores' registers are free, so that the whole row comes and goes at once.
+                uint32_t acc[D];
+                tmem_ld32_nowait(lane_base + o_col, acc);
+                tmem_ld32_nowait(lane_base + o_col + 32, acc + 32);
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < D; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
+                tmem_st32_nowait(lane_base + o_col, acc);
+                tmem_st32_nowait(lane_base + o_col + 32, acc + 32);
+                tmem_st_wait();
+            }
             fence_async_smem();
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive_cta(smem_u32(&bar_p_full[grp]));
-                mbar_arrive_cta(smem_u32(&bar_s_empty[grp]));
-            }
+            if (lane == 0) mbar_arrive_cta(smem_u32(&bar_p_full[grp]));
         }
         // the group's output, once its last product is in
         float o[D];
