@@ -82,6 +82,16 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     return warp_sum(t);
 }
 
+// The same where no earlier sum of the kernel has used `scratch`: one barrier instead of two.
+__device__ __forceinline__ float block_sum_first(float v, float* scratch) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    v = warp_sum(v);
+    if (lane == 0) scratch[warp] = v;
+    __syncthreads();
+    const int warps = (blockDim.x + 31) >> 5;
+    return warp_sum(lane < warps ? scratch[lane] : 0.0f);
+}
+
 // Which keys j <= pos a query at position pos sees, as one number: 0: all of them; W > 0: those with pos - j < W (a
 // sliding window); W < 0: those in the query's own block of -W positions, blocks counted from the sequence's position 0.
 __device__ __forceinline__ int xs_first_visible(int pos, int window) {
@@ -149,6 +159,37 @@ static inline int ceil_div_i(int64_t a, int64_t b) { return (int)((a + b - 1) / 
 // and nothing at all is written to global memory, before pdl_wait(). Without the attribute both
 // calls do nothing.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Loads of what another kernel of the step has written, in kernels that also load before the wait: a load through a `const __restrict__`
+// pointer counts as one of constant memory, which the compiler may move in front of the wait to the others.
+__device__ __forceinline__ uint4 ld_written16(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint2 ld_written8(const void* p) {
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ld_written4(const float* p) {
+    const uint4 v = ld_written16(p);
+    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
+__device__ __forceinline__ float4 ld_written4(const __nv_bfloat16* p) {
+    const uint2 v = ld_written8(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ float ld_written1(const __nv_bfloat16* p) {
+    unsigned short v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+    return __bfloat162float(__ushort_as_bfloat16(v));
+}
+__device__ __forceinline__ float ld_written1(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::); }
 
 extern int g_xs_pdl;   // 1: launches carry the attribute (xs_set_pdl)

@@ -108,14 +108,12 @@ __global__ void moe_logits_kernel(const T* __restrict__ x, int64_t ldx, const T*
     const int t = (int)(pair / E), e = (int)(pair % E);
     const T* xr = x + (int64_t)t * ldx;
     const T* we = w + (int64_t)e * K;
-    pdl_wait();
     float acc = 0.0f;
     if (vec) {          // bfloat16 rows in whole 16-byte pieces
         const uint4* x8 = reinterpret_cast<const uint4*>(xr);
         const uint4* w8 = reinterpret_cast<const uint4*>(we);
-#pragma unroll 4
-        for (int i = lane; i < (K >> 3); i += 32) {
-            const uint4 a = x8[i], b = w8[i];
+        const int pieces = K >> 3;
+        auto add = [&](const uint4& a, const uint4& b) {
             const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
             const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
 #pragma unroll
@@ -124,8 +122,23 @@ __global__ void moe_logits_kernel(const T* __restrict__ x, int64_t ldx, const T*
                 acc = fmaf(af.x, bf.x, acc);
                 acc = fmaf(af.y, bf.y, acc);
             }
-        }
+        };
+        // the router row's first 2,048 elements before the wait for the kernel that writes x, x's all in flight behind it (8 tokens, 16
+        // experts in a chain of decode kernels: 3.6 -> 2.6 us)
+        constexpr int kAhead = 8;
+        uint4 b[kAhead], a[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) b[j] = lane + 32 * j < pieces ? w8[lane + 32 * j] : make_uint4(0u, 0u, 0u, 0u);
+        pdl_wait();
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) a[j] = lane + 32 * j < pieces ? ld_written16(x8 + lane + 32 * j) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+            if (lane + 32 * j < pieces) add(a[j], b[j]);
+#pragma unroll 4
+        for (int i = lane + 32 * kAhead; i < pieces; i += 32) add(ld_written16(x8 + i), w8[i]);
     } else {
+        pdl_wait();
 #pragma unroll 8
         for (int k = lane; k < K; k += 32) acc = fmaf(to_f32(xr[k]), to_f32(we[k]), acc);
     }

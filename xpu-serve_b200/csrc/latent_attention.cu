@@ -96,8 +96,8 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
 // dst[i..i+8) and dst[i + half..) from src's two pieces, turned by cs[i..i+8) (cos, sin)
 __device__ __forceinline__ void rotate_pieces(const __nv_bfloat16* src, __nv_bfloat16* dst, const float2* cs, int i, int half) {
     float lo[8], hi[8], a[8], b[8];
-    unpack8(*reinterpret_cast<const uint4*>(src + i), lo);
-    unpack8(*reinterpret_cast<const uint4*>(src + i + half), hi);
+    unpack8(ld_written16(src + i), lo);
+    unpack8(ld_written16(src + i + half), hi);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const float2 t = cs[i + j];
@@ -108,6 +108,8 @@ __device__ __forceinline__ void rotate_pieces(const __nv_bfloat16* src, __nv_bfl
     *reinterpret_cast<uint4*>(dst + i + half) = pack8(b);
 }
 
+// (8 tokens of 16 heads in a chain of decode kernels: 4.3 -> 3.3 us with the row's place and the norm's weight before the wait and
+// the rotations in front of the sum's barrier)
 __global__ void latent_prepare_vec_kernel(const __nv_bfloat16* __restrict__ down, int64_t ld_down, const __nv_bfloat16* __restrict__ q,
                                           int64_t ld_q, const float* __restrict__ norm_w, const float2* __restrict__ table,
                                           const int32_t* __restrict__ positions, const int32_t* __restrict__ seq_of_token,
@@ -122,35 +124,34 @@ __global__ void latent_prepare_vec_kernel(const __nv_bfloat16* __restrict__ down
     const float2* cs = table != nullptr ? table + (int64_t)pos * half : nullptr;
     const int pairs = cs != nullptr ? half / 8 : 0;          // pieces that turn with a partner
     const int plain = Dr / 8 - 2 * pairs;                    // pieces that pass
+    const __nv_bfloat16* dr = down + (int64_t)t * ld_down;
+    __nv_bfloat16* row = nullptr;
+    float v[4][8], nw[4][8];
+    if (write_kv) {                                          // (where the row goes and the norm's weight: before the wait)
+        const int page = page_table[(int64_t)seq_of_token[t] * P + pos / page_size];
+        row = pool + ((int64_t)page * page_size + pos % page_size) * (R + Dr);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int c = (threadIdx.x + u * blockDim.x) * 8;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) nw[u][j] = c < R ? norm_w[c + j] : 0.0f;
+        }
+    }
     pdl_wait();
+    float ss = 0.0f;
     if (write_kv) {
-        const __nv_bfloat16* dr = down + (int64_t)t * ld_down;
-        float v[4][8];
-        float ss = 0.0f;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int c = (threadIdx.x + u * blockDim.x) * 8;
             if (c < R) {
-                unpack8(*reinterpret_cast<const uint4*>(dr + c), v[u]);
+                unpack8(ld_written16(dr + c), v[u]);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) ss += v[u][j] * v[u][j];
             }
         }
-        const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)R + eps);
-        const int page = page_table[(int64_t)seq_of_token[t] * P + pos / page_size];
-        __nv_bfloat16* row = pool + ((int64_t)page * page_size + pos % page_size) * (R + Dr);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int c = (threadIdx.x + u * blockDim.x) * 8;
-            if (c < R) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) v[u][j] = v[u][j] * inv * norm_w[c + j];
-                *reinterpret_cast<uint4*>(row + c) = pack8(v[u]);
-            }
-        }
         for (int i = threadIdx.x; i < pairs + plain; i += blockDim.x) {
             if (i < pairs) rotate_pieces(dr + R, row + R, cs, i * 8, half);
-            else *reinterpret_cast<uint4*>(row + R + dims + (i - pairs) * 8) = *reinterpret_cast<const uint4*>(dr + R + dims + (i - pairs) * 8);
+            else *reinterpret_cast<uint4*>(row + R + dims + (i - pairs) * 8) = ld_written16(dr + R + dims + (i - pairs) * 8);
         }
     }
     const int per_head = pairs + plain;
@@ -159,7 +160,19 @@ __global__ void latent_prepare_vec_kernel(const __nv_bfloat16* __restrict__ down
         const __nv_bfloat16* src = q + (int64_t)t * ld_q + (int64_t)h * (Dn + Dr) + Dn;
         __nv_bfloat16* dst = q_rot + ((int64_t)t * H + h) * Dr;
         if (i < pairs) rotate_pieces(src, dst, cs, i * 8, half);
-        else *reinterpret_cast<uint4*>(dst + dims + (i - pairs) * 8) = *reinterpret_cast<const uint4*>(src + dims + (i - pairs) * 8);
+        else *reinterpret_cast<uint4*>(dst + dims + (i - pairs) * 8) = ld_written16(src + dims + (i - pairs) * 8);
+    }
+    if (write_kv) {                                          // the sum last: the rotations' loads are not behind its barrier
+        const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)R + eps);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int c = (threadIdx.x + u * blockDim.x) * 8;
+            if (c < R) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[u][j] = v[u][j] * inv * nw[u][j];
+                *reinterpret_cast<uint4*>(row + c) = pack8(v[u]);
+            }
+        }
     }
 }
 

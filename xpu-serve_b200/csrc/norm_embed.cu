@@ -262,15 +262,25 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
     *reinterpret_cast<uint2*>(p) = raw;
 }
 
+// (Few rows: all it does is wait. The norms' weights are asked for before the wait for the previous kernel, and each sum has a place of its
+// own: 5 rows of 1,024 in a chain of decode kernels, branch norm and norm, 3.0 -> 2.4 us.)
 template <typename TM, typename TY, int NV>
 __global__ void add_rmsnorm_vec_kernel(float* __restrict__ h, const TM* __restrict__ m,
                                        const float* __restrict__ post_w, const float* __restrict__ w,
                                        TY* __restrict__ y, const int32_t* __restrict__ rows, int H, float eps_post,
                                        float eps) {
-    __shared__ float scratch[32];
+    __shared__ float scratch[2][32];
     pdl_launch_dependents();
-    pdl_wait();
     const int i = blockIdx.x;
+    float4 pw[NV], ww[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int c = threadIdx.x + k * blockDim.x;
+        const bool there = c < (H >> 2);
+        pw[k] = there && post_w != nullptr ? load4<float>(post_w + 4 * c) : make_float4(1.f, 1.f, 1.f, 1.f);
+        ww[k] = there && w != nullptr ? load4<float>(w + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    pdl_wait();
     const int64_t r = rows ? rows[i] : i;
     float* hr = h + r * H;
     const int chunks = H >> 2;
@@ -279,7 +289,7 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ h, const TM* __restri
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         const int c = threadIdx.x + k * blockDim.x;
-        v[k] = c < chunks ? load4<float>(hr + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[k] = c < chunks ? ld_written4(hr + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (m != nullptr) {
         const TM* mr = m + r * H;
@@ -288,25 +298,23 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ h, const TM* __restri
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             const int c = threadIdx.x + k * blockDim.x;
-            b[k] = c < chunks ? load4<TM>(mr + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            b[k] = c < chunks ? ld_written4(mr + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
             bs += b[k].x * b[k].x + b[k].y * b[k].y + b[k].z * b[k].z + b[k].w * b[k].w;
         }
         float inv = 1.0f;
         if (post_w != nullptr) {
-            bs = block_sum(bs, scratch);
+            bs = block_sum_first(bs, scratch[0]);
             inv = 1.0f / sqrtf(bs / (float)H + eps_post);
         }
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             const int c = threadIdx.x + k * blockDim.x;
             if (c >= chunks) continue;
-            float4 pw = make_float4(1.f, 1.f, 1.f, 1.f);
-            if (post_w != nullptr) pw = load4<float>(post_w + 4 * c);
             if (post_w != nullptr) {
-                v[k].x += b[k].x * inv * pw.x;
-                v[k].y += b[k].y * inv * pw.y;
-                v[k].z += b[k].z * inv * pw.z;
-                v[k].w += b[k].w * inv * pw.w;
+                v[k].x += b[k].x * inv * pw[k].x;
+                v[k].y += b[k].y * inv * pw[k].y;
+                v[k].z += b[k].z * inv * pw[k].z;
+                v[k].w += b[k].w * inv * pw[k].w;
             } else {
                 v[k].x += b[k].x;
                 v[k].y += b[k].y;
@@ -329,15 +337,14 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ h, const TM* __restri
     }
 #pragma unroll
     for (int k = 0; k < NV; ++k) ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
-    ss = block_sum(ss, scratch);
+    ss = block_sum_first(ss, scratch[1]);
     const float inv = 1.0f / sqrtf(ss / (float)H + eps);
     TY* yr = y + (int64_t)i * H;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         const int c = threadIdx.x + k * blockDim.x;
         if (c >= chunks) continue;
-        const float4 ww = load4<float>(w + 4 * c);
-        store4(yr + 4 * c, make_float4(v[k].x * inv * ww.x, v[k].y * inv * ww.y, v[k].z * inv * ww.z, v[k].w * inv * ww.w));
+        store4(yr + 4 * c, make_float4(v[k].x * inv * ww[k].x, v[k].y * inv * ww[k].y, v[k].z * inv * ww[k].z, v[k].w * inv * ww[k].w));
     }
 }
 
