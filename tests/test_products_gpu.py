@@ -411,6 +411,31 @@ def test_streamed_experts_at_their_lines(T, top, E, N, K):
 
 
 # ------------------------------------------------------------------------- kernels of the recurrent and latent layers
+@pytest.mark.parametrize("lens", [[1], [64, 65, 1, 700], [130] * 5])
+@pytest.mark.parametrize("H,R,Dr,window", [(16, 512, 64, 0), (3, 128, 32, 100), (16, 64, 0, 64), (5, 512, 64, 0)])
+def test_latent_attention_of_single_tokens_in_parts(lens, H, R, Dr, window):
+    """As many parts as pages, fewer, and more than there are: those without a page write nothing. Weights and outputs are
+    bfloat16: about 2^-8 of the norm."""
+    n, W = len(lens), R + Dr
+    pages = [-(-l // 64) for l in lens]
+    pool = torch.randn(sum(pages), 1, 1, 64, W, device=DEV).to(BF)
+    table, order, at = torch.full((n, max(pages) + 1), -1, dtype=torch.int32), torch.randperm(sum(pages)).to(torch.int32), 0
+    for i, c in enumerate(pages):
+        table[i, :c], at = order[at:at + c], at + c
+    ql, qr = torch.randn(n, H, R, device=DEV).to(BF), torch.randn(n, H, Dr, device=DEV).to(BF)
+    cu, kv = (torch.tensor(a, dtype=torch.int32, device=DEV) for a in (range(n + 1), lens))
+    sink = torch.rand(H, device=DEV)
+    for splits in (1, 2, 3, 11, 64):
+        out = torch.full((n, H, R), math.nan, device=DEV, dtype=BF)
+        scratch = torch.full((max(1, ops().latent_attention_mma_scratch_bytes(n * H, R, splits)),), 255, dtype=torch.uint8, device=DEV)
+        ops().latent_attention_mma(ql, qr, pool, table.to(DEV), cu, kv, None, sink, out, scratch, n, 1, 64, W ** -0.5, window, splits)
+        for i, l in enumerate(lens):
+            keys = pool[table[i, :pages[i]].long().to(DEV), 0, 0].reshape(-1, W)[max(0, l - window) if window else 0:l].double()
+            sc = torch.cat([torch.cat([ql[i], qr[i]], -1).double() @ keys.T * W ** -0.5, sink.double()[:, None]], 1)
+            ref = sc.softmax(-1)[:, :-1] @ keys[:, :R]
+            assert ((out[i].double() - ref).norm() / ref.norm()).item() < 2.0 ** -7, (splits, i)
+
+
 @pytest.mark.parametrize("B,M,N,K", [(1, 1, 1, 8), (16, 8, 512, 128), (3, 9, 33, 520), (2, 16, 31, 1032), (4, 5, 100, 24)])
 def test_batched_product_of_few_rows(B, M, N, K):
     x = torch.randn(M, B, K + 8, device=DEV).to(BF).transpose(0, 1)[:, :, :K]

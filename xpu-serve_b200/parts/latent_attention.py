@@ -147,9 +147,10 @@ class LatentAttentionMixer(Mixer):
             blocks = -(-step.max_kv_len // step.page_size)
             if s.window > 0:
                 blocks = min(blocks, -(-(s.window + step.max_q_len) // step.page_size) + 1)
-            # (at least two pages a CTA: measured on B200, 8 sequences of 2,100 keys, 16 heads of 576: 9 to 33 parts 32 to 34 us,
-            # 37 parts 40 us, 4 parts 54 us: past a page or two a CTA, more parts only add to what the combine reads)
-            splits = max(1, min(-(-blocks // 2), 64, slots // max(tiles, 1)))
+            # (a page a CTA where all fit at once: a page's rows are asked for before the wait for the kernels in front, the next page's
+            # only behind the first's products. Measured on B200, 16 heads of 576, with the combine, us: 8 sequences of 300 to 2,100
+            # keys 18.6 in half as many parts, 15.5 so; one of 2,100 14.0 and 12.4; 12 of 100 keys 10.2 in one part, 9.0 in two)
+            splits = max(1, min(blocks, 64, slots // max(tiles, 1)))
             scratch = None
             if splits > 1:
                 need = ops.latent_attention_mma_scratch_bytes(q_rot.shape[0] * s.heads, s.kv_rank, splits)
