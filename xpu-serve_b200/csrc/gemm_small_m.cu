@@ -715,8 +715,23 @@ XS_API int xs_gemm_small_m_ksplit(int M, int N, int K, int sms) {
     // that the unpredicated instances take (whole pairs of k blocks) where there are such.
     const int tiles = ceil_div_i(N, ROWS);
     if (tiles >= 2 * sms) return 1;
+    // Outputs so narrow that four slices leave half of the device's CTA slots empty take up to eight, of at least 768: chain of a 350M
+    // layer's four products, batch 1, 4 and 8, us a layer (N 1024, K 6656 in two, four and eight slices): 18.3, 16.7, 16.0; 18.7, 16.8,
+    // 16.2; 18.9, 16.9, 16.7. With 9 to 16 rows a CTA holds more registers and fetches as much of x as of the weight: as many slices as
+    // keep all CTAs resident at once, two an SM where a slice is a multiple of 2,048 (sixteen loads a round), else three. Batch 16, us a
+    // layer: N 2048, K 8192 in two and four slices 37.7, 39.9; K 10752 in two, three, four and six 48.7, 47.8, 50.2, 48.5; N 1024,
+    // K 6656 in two, four and eight 23.8, 20.9, 23.0.
+    const bool narrow = 2 * tiles <= sms;
     int ks = K / 2048;                // at least 2048 of K a slice
     if (ks > g_small_m_ksplit_max) ks = g_small_m_ksplit_max;
+    if (M <= 8 && narrow && K > 2048) ks = K / 768 < 8 ? K / 768 : 8;
+    if (M > 8) {
+        ks = 1;
+        if (N % ROWS == 0)
+            for (int k2 = 2; k2 <= 8 && K / k2 >= 1024; ++k2)
+                if (K % k2 == 0 && (K / k2) % 64 == 0 && (int64_t)tiles * k2 <= ((K / k2) % (2 * K_PER_CTA) == 0 ? 2 : 3) * (int64_t)sms) ks = k2;
+        return ks;
+    }
     while (ks > 1 && (int64_t)tiles * ks > 4 * (int64_t)sms) --ks;
     if (ks < 1) ks = 1;
     if (N % ROWS == 0)

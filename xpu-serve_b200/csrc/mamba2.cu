@@ -415,8 +415,8 @@ void launch_step(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
 // Carries the state from chunk to chunk: for each (sequence, head), S = the sequence's state; for its chunks in order,
 // the chunk's scratch state is replaced by S (where the chunk starts) and S = decay * S + (what the chunk added). The
 // final S is the sequence's state after the step. first_chunk: [n_seqs + 1].
-__global__ void mamba2_carry_kernel(float* __restrict__ state, float* __restrict__ chunk_state,
-                                    const float* __restrict__ chunk_decay, const int32_t* __restrict__ first_chunk,
+__global__ void mamba2_carry_kernel(float* __restrict__ state, float* chunk_state,
+                                    const float* chunk_decay, const int32_t* __restrict__ first_chunk,
                                     const int32_t* __restrict__ slots, int heads, int64_t NP) {
     pdl_launch_dependents();
     const int h = blockIdx.x, seq = blockIdx.y;
@@ -425,11 +425,21 @@ __global__ void mamba2_carry_kernel(float* __restrict__ state, float* __restrict
     pdl_wait();
     for (int64_t i = (int64_t)blockIdx.z * blockDim.x + threadIdx.x; i < NP; i += (int64_t)gridDim.z * blockDim.x) {
         float S = st[i];
-        for (int c = c_lo; c < c_hi; ++c) {
-            float* cs = chunk_state + ((int64_t)c * heads + h) * NP + i;
-            const float added = *cs;
-            *cs = S;
-            S = fmaf(chunk_decay[(int64_t)c * heads + h], S, added);
+        // (eight chunks' states and decays asked for together: one after another each waited for memory on its own)
+        for (int c0 = c_lo; c0 < c_hi; c0 += 8) {
+            float added[8], decay[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const bool there = c0 + j < c_hi;
+                added[j] = there ? chunk_state[((int64_t)(c0 + j) * heads + h) * NP + i] : 0.0f;
+                decay[j] = there ? chunk_decay[(int64_t)(c0 + j) * heads + h] : 0.0f;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (c0 + j >= c_hi) break;
+                chunk_state[((int64_t)(c0 + j) * heads + h) * NP + i] = S;
+                S = fmaf(decay[j], S, added[j]);
+            }
         }
         st[i] = S;
     }

@@ -251,9 +251,11 @@ mlstm_scan_kernel(const TX* __restrict__ qkv, int64_t ld, int q_col, int k_col, 
 //     m' = max(m + F, m_loc);   S' = exp(m + F - m') S + exp(m_loc - m') S_loc;   n' likewise
 // which is what the token-by-token recurrence gives (its maximum unrolls to exactly this). Afterwards the slot holds the
 // state behind the step's last token.
-__global__ void mlstm_carry_kernel(float* __restrict__ s_state, float* __restrict__ nm_state, float* __restrict__ s_chunk,
-                                   float* __restrict__ nm_chunk, const int32_t* __restrict__ first_chunk,
+// (The maxima run ahead of the entries, which stay in registers over the chunks; eight chunks' entries are asked for together.)
+__global__ void mlstm_carry_kernel(float* s_state, float* nm_state, float* s_chunk, float* nm_chunk, const int32_t* __restrict__ first_chunk,
                                    const int32_t* __restrict__ slots, int H, int D, int Dv, int Z) {
+    constexpr int kRun = 128;                             // chunks at a time
+    __shared__ float loc_s[kRun], f_s[kRun], before_s[kRun], after_s[kRun], ca_s[kRun], cb_s[kRun];
     pdl_launch_dependents();
     const int seq = blockIdx.x, head = blockIdx.y;
     const int64_t slot = slots[seq];
@@ -262,29 +264,56 @@ __global__ void mlstm_carry_kernel(float* __restrict__ s_state, float* __restric
     float* S = s_state + ((slot * H + head) * D) * (int64_t)Dv;
     float* nm = nm_state + (slot * H + head) * (int64_t)Z * (D + 1);
     const int n_s = D * Dv, n_n = Z * D;
+    const int64_t s_step = (int64_t)H * D * Dv, n_step = (int64_t)H * Z * (D + 2);
     float m = nm[D];                                      // (every copy holds the same m)
-    for (int j = j0; j < j1; ++j) {
-        float* Sl = s_chunk + (((int64_t)j * H + head) * D) * (int64_t)Dv;
-        float* nml = nm_chunk + ((int64_t)j * H + head) * (int64_t)Z * (D + 2);
-        const float m_loc = nml[D], F = nml[D + 1];
-        const float m_new = fmaxf(m + F, m_loc);
-        const float ca = expf(m + F - m_new), cb = expf(m_loc - m_new);
-        __syncthreads();                                  // every thread has read the chunk's m and F
-        for (int e = threadIdx.x; e < n_s; e += blockDim.x) {
-            const float loc = Sl[e], run = S[e];
-            Sl[e] = run;
-            S[e] = ca * run + cb * loc;
-        }
-        for (int e = threadIdx.x; e < n_n; e += blockDim.x) {
-            const int z = e / D, d = e - z * D;
-            const float loc = nml[z * (D + 2) + d], run = nm[z * (D + 1) + d];
-            nml[z * (D + 2) + d] = run;
-            nm[z * (D + 1) + d] = ca * run + cb * loc;
+    for (int jb = j0; jb < j1; jb += kRun) {
+        const int run = min(kRun, j1 - jb);
+        float* Sl = s_chunk + (((int64_t)jb * H + head) * D) * (int64_t)Dv;
+        float* nml = nm_chunk + ((int64_t)jb * H + head) * (int64_t)Z * (D + 2);
+        __syncthreads();
+        for (int j = threadIdx.x; j < run; j += blockDim.x) {
+            loc_s[j] = nml[j * n_step + D];
+            f_s[j] = nml[j * n_step + D + 1];
         }
         __syncthreads();
-        if ((int)threadIdx.x < Z) nml[threadIdx.x * (D + 2) + D] = m;       // the chunk starts from this m
-        m = m_new;
+        if (threadIdx.x == 0) {
+            float at = m;
+            for (int j = 0; j < run; ++j) {
+                before_s[j] = at;
+                at = fmaxf(at + f_s[j], loc_s[j]);
+                after_s[j] = at;
+            }
+        }
+        __syncthreads();
+        m = after_s[run - 1];
+        for (int j = threadIdx.x; j < run; j += blockDim.x) {
+            ca_s[j] = expf(before_s[j] + f_s[j] - after_s[j]);
+            cb_s[j] = expf(loc_s[j] - after_s[j]);
+        }
+        __syncthreads();
+        auto walk = [&](float* state, float* chunk, int64_t step) {
+            float at = *state;
+            for (int j = 0; j < run; j += 8) {
+                float loc[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) loc[u] = j + u < run ? chunk[(j + u) * step] : 0.0f;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    if (j + u >= run) break;
+                    chunk[(j + u) * step] = at;
+                    at = ca_s[j + u] * at + cb_s[j + u] * loc[u];
+                }
+            }
+            *state = at;
+        };
+        for (int e = threadIdx.x; e < n_s; e += blockDim.x) walk(S + e, Sl + e, s_step);
+        for (int e = threadIdx.x; e < n_n; e += blockDim.x) {
+            const int z = e / D, d = e - z * D;
+            walk(nm + z * (D + 1) + d, nml + z * (D + 2) + d, n_step);
+        }
+        for (int i = threadIdx.x; i < run * Z; i += blockDim.x) nml[(i / Z) * n_step + (i % Z) * (D + 2) + D] = before_s[i / Z];   // the chunk starts from this m
     }
+    __syncthreads();
     if ((int)threadIdx.x < Z) nm[threadIdx.x * (D + 1) + D] = m;
 }
 
@@ -299,11 +328,12 @@ XS_API int xs_mlstm_copies(int Dv) { return (Dv + COLS - 1) / COLS; }
 // With a chunk list (chunks [n_chunks, 3]: sequence, first token, tokens; first_chunk [n_seqs + 1]; s_chunk [n_chunks, H, D, Dv]
 // and nm_chunk [n_chunks, H, Z, D + 2] float32 scratch) the chunks run side by side: a pass from the empty state that leaves
 // each chunk's end state, a carry over each sequence's chunks in order, and a pass from each chunk's true state that writes y
-// (three launches, twice the recurrence's work, a sequence's tokens no longer one after another).
+// (three launches, twice the recurrence's work, a sequence's tokens no longer one after another). single: every sequence brings one
+// token, and the kernel's buffers are of one token (the same sums in the same order, without the loops over absent tokens).
 XS_API int xs_mlstm_scan(const void* qkv, int64_t ld, int q_col, int k_col, int v_col, const float* gates, int64_t ldg,
                          const float* i_bias, const float* f_bias, float* s_state, float* nm_state, const int32_t* cu_seqlens,
                          const int32_t* slots, float* y, int n_seqs, int H, int D, int Dv, float cap, float q_scale, int dtype,
-                         const int32_t* chunks, const int32_t* first_chunk, int n_chunks, float* s_chunk, float* nm_chunk,
+                         const int32_t* chunks, const int32_t* first_chunk, int n_chunks, float* s_chunk, float* nm_chunk, int single,
                          cudaStream_t stream) {
     if (n_seqs == 0) return 0;
     XS_REQUIRE(n_seqs > 0 && H > 0 && D > 0 && Dv > 0 && cap > 0.0f, "mlstm: %d sequences, %d heads of %d and %d, cap %g", n_seqs, H,
@@ -318,8 +348,9 @@ XS_API int xs_mlstm_scan(const void* qkv, int64_t ld, int q_col, int k_col, int 
     int mode = chunked ? 1 : 0;
     const int blocks = Dv >= COLS ? MAX_CW : (Dv + 31) / 32;      // blocks of 32 columns in a CTA (all CTAs alike)
     const int threads = 32 * (1 + blocks * RG);
-#define XS_GO(TT, DP)                                                                                                  \
-    xs_launch(mlstm_scan_kernel<TT, DP, (DP <= 128 ? 8 : 4)>, grid, dim3(threads), 0, stream, (const TT*)qkv, ld, q_col, k_col, v_col, gates,  \
+#define XS_GO(TT, DP) do { if (single && !chunked) XS_GO_CH(TT, DP, 1); else XS_GO_CH(TT, DP, (DP <= 128 ? 8 : 4)); } while (0)
+#define XS_GO_CH(TT, DP, CH)                                                                                           \
+    xs_launch(mlstm_scan_kernel<TT, DP, CH>, grid, dim3(threads), 0, stream, (const TT*)qkv, ld, q_col, k_col, v_col, gates,  \
               ldg, i_bias, f_bias, s_state, nm_state, cu_seqlens, slots, y, H, D, Dv, cap, q_scale, chunks, mode, s_chunk, nm_chunk)
 #define XS_BY_D(TT)                      \
     do {                                 \
@@ -332,7 +363,7 @@ XS_API int xs_mlstm_scan(const void* qkv, int64_t ld, int q_col, int k_col, int 
     XS_DISPATCH_DTYPE(dtype, TT, XS_BY_D(TT));
     XS_LAUNCH_CHECK("mlstm_scan");
     if (chunked) {
-        xs_launch(mlstm_carry_kernel, dim3(n_seqs, H), dim3(256), 0, stream, s_state, nm_state, s_chunk, nm_chunk, first_chunk,
+        xs_launch(mlstm_carry_kernel, dim3(n_seqs, H), dim3(1024), 0, stream, s_state, nm_state, s_chunk, nm_chunk, first_chunk,
                   slots, H, D, Dv, Z);
         XS_LAUNCH_CHECK("mlstm_carry");
         mode = 2;
@@ -341,5 +372,6 @@ XS_API int xs_mlstm_scan(const void* qkv, int64_t ld, int q_col, int k_col, int 
     }
 #undef XS_BY_D
 #undef XS_GO
+#undef XS_GO_CH
     return 0;
 }

@@ -44,6 +44,23 @@ __global__ void embed_kernel(const TW* __restrict__ table, const int32_t* __rest
     for (int c = threadIdx.x; c < H; c += blockDim.x) out[c] = to_f32(row[c]) * scale;
 }
 
+// The same for bfloat16 rows on 16-byte boundaries whose width is a multiple of 8: eight elements a thread, one load.
+__global__ void embed_bf16x8_kernel(const __nv_bfloat16* __restrict__ table, const int32_t* __restrict__ ids, float* __restrict__ h, int T,
+                                    int H, float scale) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = blockIdx.x;
+    const uint4* row = reinterpret_cast<const uint4*>(table + (int64_t)ids[t] * H);
+    float4* out = reinterpret_cast<float4*>(h + (int64_t)t * H);
+    for (int c = threadIdx.x; c < (H >> 3); c += blockDim.x) {
+        const uint4 raw = row[c];
+        const __nv_bfloat162* two = reinterpret_cast<const __nv_bfloat162*>(&raw);
+        const float2 a = __bfloat1622float2(two[0]), b = __bfloat1622float2(two[1]), e = __bfloat1622float2(two[2]), f = __bfloat1622float2(two[3]);
+        out[2 * c] = make_float4(a.x * scale, a.y * scale, b.x * scale, b.y * scale);
+        out[2 * c + 1] = make_float4(e.x * scale, e.y * scale, f.x * scale, f.y * scale);
+    }
+}
+
 // A token's row plus a row of a second table chosen by a hash of the previous and the current token, plus a sine/cosine
 // vector of the position, then an RMS norm (w == nullptr: none):
 //     x = table[tok] * scale + pair[pos == 0 ? buckets : (prev * mul_prev + tok * mul_cur) mod buckets]
@@ -124,6 +141,11 @@ XS_API int xs_embed(const void* table, int table_dtype, const int32_t* ids, floa
                     cudaStream_t stream) {
     if (T == 0) return 0;
     XS_REQUIRE(T > 0 && H > 0, "embed: %d tokens of width %d", T, H);
+    if (table_dtype == XS_BF16 && H % 8 == 0 && ((uintptr_t)table | (uintptr_t)h) % 16 == 0) {
+        xs_launch(embed_bf16x8_kernel, dim3(T), dim3(H >= 1024 ? 256 : 128), 0, stream, (const __nv_bfloat16*)table, ids, h, T, H, scale);
+        XS_LAUNCH_CHECK("embed");
+        return 0;
+    }
     XS_DISPATCH_DTYPE(table_dtype, TW,
                       xs_launch(embed_kernel<TW>, dim3(T), dim3(256), 0, stream, (const TW*)table, ids, h, T, H, scale));
     XS_LAUNCH_CHECK("embed");

@@ -76,7 +76,7 @@ def _signatures(lib) -> None:
         "xs_moe_few_rows": [P, L, I, P, P, L, P, I, I, I, I, I, I, F, F, F, P],
         "xs_relu_squared": [P, P, I, L, P],
         "xs_embed_pair": [P, P, I, P, P, P, P, P, P, P, P, P, I, I, F, I, ctypes.c_longlong, ctypes.c_longlong, F, P],
-        "xs_mlstm_scan": [P, L, I, I, I, P, L, P, P, P, P, P, P, P, I, I, I, I, F, F, I, P, P, I, P, P, P],
+        "xs_mlstm_scan": [P, L, I, I, I, P, L, P, P, P, P, P, P, P, I, I, I, I, F, F, I, P, P, I, P, P, I, P],
         "xs_latent_prepare": [P, L, P, L, P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, F, I, I, P],
         "xs_latent_attention_generic": [P, L, L, P, P, P, I, P, P, P, L, P, P, L, L, I, I, I, I, I, F, I, I, P],
         "xs_gemm_batched": [P, L, L, P, L, L, P, L, L, I, I, I, I, I, P],
@@ -1221,7 +1221,7 @@ def mlstm_scan(qkv: torch.Tensor, q_col: int, k_col: int, v_col: int, gates: tor
     _check(load().xs_mlstm_scan(qkv.data_ptr(), qkv.stride(0), int(q_col), int(k_col), int(v_col), gates.data_ptr(),
                                 gates.stride(0), i_bias.data_ptr(), f_bias.data_ptr(), s_state.data_ptr(), nm_state.data_ptr(),
                                 cu_seqlens.data_ptr(), slots.data_ptr(), y.data_ptr(), cu_seqlens.numel() - 1, heads, dim, vdim,
-                                float(cap), float(q_scale), _code(qkv), *chunk_args, _stream()),
+                                float(cap), float(q_scale), _code(qkv), *chunk_args, 1 if T == cu_seqlens.numel() - 1 else 0, _stream()),
            kernels=3 if chunks is not None else 1)
 
 
