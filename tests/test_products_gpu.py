@@ -30,7 +30,7 @@ def f32_limit(K):
 # ------------------------------------------------------------------------------------------- float32 product
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (1, 8, 32), (3, 7, 36), (4, 9, 1024), (5, 1030, 1028), (8, 40, 2052), (9, 15, 1020),
                                    (16, 2500, 96), (17, 33, 64), (40, 4736, 40), (63, 65, 100), (64, 4800, 33), (65, 64, 32),
-                                   (130, 129, 68), (200, 56900, 16)])
+                                   (130, 129, 68), (200, 56900, 16), (224, 1024, 36), (225, 1024, 36), (300, 2048, 64), (700, 2050, 40)])
 def test_float32_product(M, N, K):
     ld = (K + 3) // 4 * 4 + 4
     x = torch.randn(M, ld, device=DEV)[:, :K]

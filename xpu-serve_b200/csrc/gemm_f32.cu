@@ -13,22 +13,27 @@
 //     (With 128 threads, stages of 512 k and one or two weight rows a thread the SM had one warp a scheduler: 2.0 TB/s.)
 //   more rows: bound by the FMA units. 64 x 128 outputs a CTA of 128 threads, 8 x 8 a thread, both operands in stages of 32 k as
 //     they lie in memory (rows of k, 36 floats apart: the eight rows of a 16-byte load's phase fall into different banks), so
-//     nothing is transposed; a stage is exactly one partial.
+//     nothing is transposed; a stage is exactly one partial. Where such tiles are few for the device's SMs, 64 x 64 a CTA and 4 x 8 a
+//     thread: a warp alone multiplies no more often than every second cycle, so an SM of one tile wants its outputs on more warps
+//     (one of 64 x 64 with 8 x 8 a thread took as long as one of 64 x 128: 424 us at K 6656, on four warps 270). With the device
+//     full 8 x 8 is the better one, since it reads less from shared memory a product.
 //
 // Measured on B200 (products of the 350M shape, weights from memory, us; before: the 64 x 64 tile of gemm_generic.cu, whose time
 // does not depend on the rows):
-//     N 13312 K 1024    4 rows 210 -> 13.5 (4.0 TB/s)   16 rows 212 -> 32   64 rows 221 -> 76    1,294 rows 1,569 -> 852 (41 TFLOP/s)
-//     N  1024 K 6656    4 rows 1,218 -> 14.7            16 rows 1,232 -> 20   64 rows 1,264 -> 72   1,294 rows 1,144 -> 735
+//     N 13312 K 1024    4 rows 210 -> 13.5 (4.0 TB/s)   16 rows 212 -> 32   64 rows 221 -> 76    1,294 rows 1,569 -> 832 (42 TFLOP/s)
+//     N  1024 K 6656    4 rows 1,218 -> 14.7            16 rows 1,232 -> 20   64 rows 1,264 -> 72   1,294 rows 1,144 -> 615
 //     N 65536 K 1024    4 rows 462 -> 52 (5.2 TB/s)     16 rows 464 -> 140
-// On both sides of the line between the kernels (us, L2 flushed, launch included):
-//     rows               16     64     65    128    300  1,294
-//     N 13312 K 1024     37     76    121    123    227    872     (tiles from 17 rows on)
-//     N  2048 K 1024     12     27     72     72     72    188
-//     N  1024 K 1024     10     18     72     72     72    121
-//     N  1024 K 6656     25     78    424    424    425    743
-// The line at 64 rows is right for wide outputs only. Where tiles leave most of the device idle, from 65 to some 300 rows of the
-// narrow shapes, passes of 16 rows would still be faster (K 6656: about 110 us at 96 rows); the tile there is faster than the 64 x 64
-// tile of gemm_generic.cu all the same.
+// Tiles of both kinds (us, L2 flushed; 64 x 128 of 8 x 8 / 64 x 64 of 4 x 8):
+//     rows                65          128          300          700          1,294
+//     N 13312 K 1024   117 / 102   119 / 104   225 / 254    444 / 492    832 / 907
+//     N  3072 K 1024    74 / 49     74 / 49     75 / 80     119 / 135    225 / 223
+//     N  2048 K 1024    74 / 47     74 / 47     74 / 74     117 / 102    182 / 168
+//     N  1024 K 1024    72 / 47     72 / 47     74 / 47      74 / 78     117 / 102
+//     N  1024 K 6656   424 / 270   424 / 270   436 / 272    438 / 471    709 / 615
+// n tiles on the SM that has the most take 56 n + 18 us (64 x 128) or 31 n + 16 (64 x 64) at K 1024: hence the line between them.
+// Passes of 16 rows against the 64 x 64 tiles (us): N 1024 K 1024 35 / 47 at 160 rows, 41 / 47 at 192, 51 / 47 at 256; K 6656 166 /
+// 271 at 160, 256 / 272 at 256; N 2048 K 1024 39 / 47 at 96 rows, 47 / 47 at 128, 53 / 47 at 144; N 3072 K 1024 43 / 47 at 80, 51 / 48
+// at 96: passes up to 14 x 1,024 passes times outputs a row.
 #include <atomic>
 
 #include "common.cuh"
@@ -40,6 +45,8 @@ constexpr int kStages = 3;            // of the tile kernel
 constexpr int kFewThreads = 256, kFewRows = 8;      // few rows: threads and weight rows a CTA
 constexpr int kStageK = 4 * kFewThreads;            // few rows: k of a stage, a 16-byte piece of every row a thread
 constexpr int kFewRowsMost = 64;
+constexpr int kFewOutputs = 14 * 1024;               // passes of 16 rows times outputs a row
+constexpr int kSmemOfSm = 228 * 1024; // shared memory of an SM, of which each CTA takes 1 KB for itself
 constexpr int kDevices = 64;          // devices that remember their shared-memory limit (further ones set it each time)
 
 __device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -162,16 +169,17 @@ gemm_f32_few_rows_kernel(const float* __restrict__ x, const float* __restrict__ 
 
 constexpr int BM = 64, kRow = kChunk + 4;
 
-template <int BN>
-__global__ void __launch_bounds__(BN, 256 / BN)
+// RT x 8 outputs a thread, CTAS CTAs an SM.
+template <int BN, int RT, int CTAS>
+__global__ void __launch_bounds__(BN / 8 * (BM / RT), CTAS)
 gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                      float* __restrict__ out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo) {
     extern __shared__ __align__(16) float sm[];
-    constexpr int kTileFloats = (BM + BN) * kRow, TX = BN / 8;
+    constexpr int kTileFloats = (BM + BN) * kRow, TX = BN / 8, TY = BM / RT, kStep = TX * TY / 8;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
     const int stages = (K + kChunk - 1) / kChunk;
-    // a thread copies the piece tid & 7 of the rows tid / 8, + TX, + 2 TX, ... of each operand
+    // a thread copies the piece tid & 7 of the rows tid / 8, + kStep, + 2 kStep, ... of each operand
     const int piece = threadIdx.x & 7, row = threadIdx.x >> 3;
     auto load = [&](int s, bool weights, bool inputs) {
         float* to = sm + (s % kStages) * kTileFloats;
@@ -179,18 +187,18 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
         const int left = min(16, max(0, (K - k) * 4));
         if (inputs) {
 #pragma unroll
-            for (int q = 0; q < BM / TX; ++q) {
-                const int m = m0 + row + TX * q;
+            for (int q = 0; q < BM / kStep; ++q) {
+                const int m = m0 + row + kStep * q;
                 const int n_bytes = m < M ? left : 0;
-                copy16(smem_at(to + (row + TX * q) * kRow + piece * 4), n_bytes > 0 ? x + (int64_t)m * ldx + k : x, n_bytes);
+                copy16(smem_at(to + (row + kStep * q) * kRow + piece * 4), n_bytes > 0 ? x + (int64_t)m * ldx + k : x, n_bytes);
             }
         }
         if (weights) {
 #pragma unroll
-            for (int q = 0; q < BN / TX; ++q) {
-                const int n = n0 + row + TX * q;
+            for (int q = 0; q < BN / kStep; ++q) {
+                const int n = n0 + row + kStep * q;
                 const int n_bytes = n < N ? left : 0;
-                copy16(smem_at(to + (BM + row + TX * q) * kRow + piece * 4), n_bytes > 0 ? w + (int64_t)n * ldw + k : w, n_bytes);
+                copy16(smem_at(to + (BM + row + kStep * q) * kRow + piece * 4), n_bytes > 0 ? w + (int64_t)n * ldw + k : w, n_bytes);
             }
         }
     };
@@ -204,9 +212,9 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
         if (s < stages) load(s, false, true);
         copies_commit();
     }
-    float acc[8][8];
+    float acc[RT][8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < RT; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
     for (int s = 0; s < stages; ++s) {
@@ -216,37 +224,37 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
         copies_commit();
         const float* xs = sm + (s % kStages) * kTileFloats + ty * kRow;
         const float* ws = sm + (s % kStages) * kTileFloats + (BM + tx) * kRow;
-        float part[8][8];
+        float part[RT][8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < RT; ++i)
 #pragma unroll
             for (int j = 0; j < 8; ++j) part[i][j] = 0.0f;
 #pragma unroll 2
         for (int k = 0; k < kChunk; k += 4) {
-            float4 a[8];
+            float4 a[RT];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(xs + 8 * i * kRow + k);
+            for (int i = 0; i < RT; ++i) a[i] = *reinterpret_cast<const float4*>(xs + TY * i * kRow + k);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float4 b = *reinterpret_cast<const float4*>(ws + TX * j * kRow + k);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].x, b.x, part[i][j]);
+                for (int i = 0; i < RT; ++i) part[i][j] = fmaf(a[i].x, b.x, part[i][j]);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].y, b.y, part[i][j]);
+                for (int i = 0; i < RT; ++i) part[i][j] = fmaf(a[i].y, b.y, part[i][j]);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].z, b.z, part[i][j]);
+                for (int i = 0; i < RT; ++i) part[i][j] = fmaf(a[i].z, b.z, part[i][j]);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].w, b.w, part[i][j]);
+                for (int i = 0; i < RT; ++i) part[i][j] = fmaf(a[i].w, b.w, part[i][j]);
             }
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < RT; ++i)
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[i][j] += part[i][j];
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + ty + 8 * i;
+    for (int i = 0; i < RT; ++i) {
+        const int m = m0 + ty + TY * i;
         if (m >= M) continue;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -280,15 +288,20 @@ cudaError_t launch_few(const float* x, const float* w, const float* bias, float*
                      out, M, N, K, ldx, ldw, ldo);
 }
 
-template <int BN>
+template <int BN, int RT, int CTAS>
 cudaError_t launch_tile(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int64_t ldx, int64_t ldw,
                         int64_t ldo, cudaStream_t stream) {
-    const size_t smem = (size_t)kStages * (BM + BN) * kRow * sizeof(float);
+    const size_t needs = (size_t)kStages * (BM + BN) * kRow * sizeof(float);
+    // No more CTAs an SM than an even share: the CTAs of this launch that start while the kernel before it still runs take the places
+    // that it left, which gave some SMs four tiles where three would do (N 1024, K 6656, 1,294 rows in a run of launches: 800 us
+    // instead of 616; with the limit 607).
+    const int64_t share = ((int64_t)ceil_div_i(N, BN) * ceil_div_i(M, BM) + 147) / 148;
+    const size_t fills = share < CTAS ? (size_t)(kSmemOfSm / (int)share - 1024) & ~(size_t)15 : 0, smem = fills > needs ? fills : needs;
     static std::atomic<bool> done[kDevices];
-    const cudaError_t e = opt_in(gemm_f32_tile_kernel<BN>, smem, done);
+    const cudaError_t e = opt_in(gemm_f32_tile_kernel<BN, RT, CTAS>, kSmemOfSm - 1024, done);
     if (e != cudaSuccess) return e;
-    return xs_launch(gemm_f32_tile_kernel<BN>, dim3(ceil_div_i(N, BN), ceil_div_i(M, BM)), dim3(BN), smem, stream, x, w, bias, out, M, N, K,
-                     ldx, ldw, ldo);
+    return xs_launch(gemm_f32_tile_kernel<BN, RT, CTAS>, dim3(ceil_div_i(N, BN), ceil_div_i(M, BM)), dim3(BN / 8 * (BM / RT)), smem, stream,
+                     x, w, bias, out, M, N, K, ldx, ldw, ldo);
 }
 
 }  // namespace
@@ -301,17 +314,18 @@ bool xs_gemm_f32_takes(const void* x, const void* w, int64_t ldx, int64_t ldw) {
 int xs_gemm_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int64_t ldx, int64_t ldw,
                 int64_t ldo, cudaStream_t stream) {
     cudaError_t e;
-    // (between 17 and 64 rows: the tiles where they are enough to fill half of the device's SMs)
-    if (M <= 16 || (M <= kFewRowsMost && ceil_div_i(N, 64) < 74)) {
+    // (between 17 and 64 rows: the tiles where they are enough to fill half of the device's SMs; above, passes of 16 rows of narrow
+    // products)
+    if (M <= 16 || (M <= kFewRowsMost && ceil_div_i(N, 64) < 74) || (int64_t)ceil_div_i(M, 16) * N <= kFewOutputs) {
         e = M <= 4 ? launch_few<4>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream)
             : M <= 8 ? launch_few<8>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream)
                      : launch_few<16>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream);
     } else {
         XS_REQUIRE(ceil_div_i(M, BM) <= 65535, "gemm: %d rows exceed the grid limit", M);
-        // the wide tile reads less from shared memory a product; the narrow one where it would leave less than three CTAs an SM
-        const int64_t wide = (int64_t)ceil_div_i(M, BM) * ceil_div_i(N, 128);
-        e = wide >= 3 * 148 ? launch_tile<128>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream)
-                            : launch_tile<64>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream);
+        // (tiles on the SM that has the most; the figures are above)
+        const int64_t rows = ceil_div_i(M, BM), narrow = (rows * ceil_div_i(N, 64) + 147) / 148, wide = (rows * ceil_div_i(N, 128) + 147) / 148;
+        e = 5 * narrow < 9 * wide ? launch_tile<64, 4, 4>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream)
+                                  : launch_tile<128, 8, 2>(x, w, bias, out, M, N, K, ldx, ldw, ldo, stream);
     }
     XS_REQUIRE(e == cudaSuccess, "gemm (float32): launch failed: %s", cudaGetErrorString(e));
     return 0;
