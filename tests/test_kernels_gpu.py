@@ -50,6 +50,16 @@ def test_embed(dtype):
     assert torch.equal(h, table[ids.long()].float())
 
 
+@pytest.mark.parametrize("H", [8, 1024, 2056, 203])
+def test_embed_of_rows_in_pieces_of_eight(H):
+    """Rows of bfloat16 on 16-byte boundaries and others: the products with the scale are exact in float32 up to their one rounding."""
+    table = torch.randn(33, H, device=DEV).bfloat16()
+    ids = torch.randint(0, 33, (300,), dtype=torch.int32, device=DEV)
+    h = torch.full((301, H), 7.0, device=DEV)
+    ops().embed(table, ids, h[:300], 1.7)
+    assert torch.equal(h[:300], table[ids.long()].float() * 1.7) and bool((h[300] == 7.0).all())
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H", [96, 200, 2048, 5000])
 def test_add_rmsnorm_all_forms(dtype, H):
@@ -197,7 +207,8 @@ def test_gemm_small_m(M, N, K):
 
 @pytest.mark.parametrize("M,N,K,ksplit", [(8, 2048, 8192, 4), (3, 100, 4104, 3), (16, 256, 2048, 8), (1, 48, 512, 2), (5, 2048, 2048, 7),
                                           (8, 2048, 8192, 2), (6, 1024, 6144, 3), (8, 2048, 10752, 4), (4, 512, 6656, 2),
-                                          (16, 256, 1536, 3)])
+                                          (16, 256, 1536, 3), (8, 1024, 6656, 8), (3, 1000, 6152, 8), (16, 2048, 10752, 3),
+                                          (9, 1024, 6656, 4)])
 def test_gemm_small_m_k_slices(M, N, K, ksplit):
     """K cut into slices over several CTAs: the last CTA of a tile to arrive adds the slices in slice order, so
     the bits do not depend on which one that was; a second and third call find the counters reset."""

@@ -445,7 +445,30 @@ def test_mlstm_kernel_alone(H, D, Dv, dtype):
         assert torch.equal(S[free].cpu(), S0[free]) and torch.equal(nm[free].cpu(), nm0[free])
 
 
-@pytest.mark.parametrize("H,D,Dv,chunk", [(3, 10, 14, 7), (2, 64, 70, 128), (1, 128, 32, 50), (1, 130, 70, 64)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,D,Dv", [(3, 10, 14), (2, 64, 300), (1, 128, 40), (1, 200, 40), (5, 1, 1)])
+def test_mlstm_of_single_tokens_is_the_scan(H, D, Dv, dtype):
+    """A launch of one token a sequence takes an instance of its own: outputs and states are those of the same sequences in a launch
+    with a longer one beside them, bit for bit."""
+    from xpu_serve_b200.ops import lib as ops
+    gen = torch.Generator(device="cuda").manual_seed(H * 100 + D)
+    r = lambda *shape: torch.randn(*shape, device="cuda", generator=gen)
+    seqs, Z = 5, ops.mlstm_copies(Dv)
+    proj, gates, bi, bf = r(seqs + 3, 2 * H * D + H * Dv).to(dtype), 4.0 * r(seqs + 3, 2 * H), r(H), r(H)
+    S0, nm0 = r(seqs + 2, H, D, Dv), r(seqs + 2, H, 1, D + 1).repeat(1, 1, Z, 1).contiguous()
+    slots = torch.tensor([3, 0, 6, 1, 5, 2], dtype=torch.int32, device="cuda")
+    got = []
+    for q_lens in ([1] * seqs, [1] * seqs + [3]):
+        S, nm, y = S0.clone(), nm0.clone(), torch.zeros(sum(q_lens), H * Dv, device="cuda")
+        cu = torch.tensor([0] + list(np.cumsum(q_lens)), dtype=torch.int32, device="cuda")
+        ops.mlstm_scan(proj[:sum(q_lens)], 0, H * D, 2 * H * D, gates[:sum(q_lens)], bi, bf, S, nm, cu, slots[:len(q_lens)], y, H, D,
+                       Dv, 6.0, 0.4)
+        used = slots[:seqs].long()
+        got.append((y[:seqs], S[used], nm[used]))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("H,D,Dv,chunk", [(3, 10, 14, 7), (2, 64, 70, 128), (1, 128, 32, 50), (1, 130, 70, 64), (2, 20, 14, 2)])
 def test_mlstm_kernel_in_chunks(H, D, Dv, chunk):
     """Sequences of 300, 46 and 520 tokens cut into chunks that run side by side (a pass from the empty state, the carry,
     a pass from each chunk's true state), from states that are not zero: outputs and end states against the plain

@@ -506,6 +506,40 @@ def test_mamba2_step_is_the_scan_of_one_token(heads, P, N, G, seqs, dtype):
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize("chunk,lens", [(4, [100, 3, 33]), (8, [64, 65, 8]), (1, [17, 1])])
+def test_mamba2_carry_over_many_chunks(chunk, lens):
+    """More chunks than the carry asks for at one time, and one more or fewer. Every token's update and every chunk's carry rounds once
+    against the largest state, and an output sums N products: at most T + N roundings."""
+    heads, P, N, G = 4, 12, 20, 2
+    inner, T = heads * P, sum(lens)
+    C = inner + 2 * G * N
+    r = lambda *s: torch.randn(*s, device=DEV)                                     # noqa: E731
+    xbc, proj, bias, a_log, skip = r(T, C), r(T, inner + C + heads), r(heads), r(heads) * 0.5, r(heads)
+    state = r(len(lens), heads, N, P)
+    want, states, starts, rows, first, t = [], [], [0], [], [0], 0
+    for i, n in enumerate(lens):
+        rows += [(i, t + k, min(chunk, n - k)) for k in range(0, n, chunk)]
+        first.append(len(rows))
+        s = state[i].double()
+        for _ in range(n):
+            x = xbc[t].double()[:inner].view(heads, P)
+            Bm, Cm = (m.view(G, N).repeat_interleave(heads // G, 0) for m in xbc[t].double()[inner:].split(G * N))
+            dt = torch.nn.functional.softplus(proj[t].double()[inner + C:] + bias.double())
+            s = s * torch.exp(-torch.exp(a_log.double()) * dt)[:, None, None] + (dt[:, None] * Bm)[..., None] * x[:, None]
+            y = ((s * Cm[..., None]).sum(1) + skip.double()[:, None] * x).reshape(inner)
+            want.append(y * torch.nn.functional.silu(proj[t].double()[:inner]))
+            t += 1
+        starts.append(t)
+        states.append(s)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)                # noqa: E731
+    out = torch.empty(T, inner, device=DEV)
+    ops().mamba2_scan(xbc, proj, inner + C, bias, a_log, skip, state, i32(starts), i32(range(len(lens))), out, heads, P, N, G,
+                      chunks=(i32(rows), i32(first), torch.empty(len(rows), heads, N, P, device=DEV),
+                              torch.empty(len(rows), heads, device=DEV)))
+    limit = (max(lens) + N) * 2.0 ** -24
+    assert gap(out, torch.stack(want)) <= limit and gap(state, torch.stack(states)) <= limit
+
+
 def test_mamba2_step_of_more_tokens_than_sequences_is_refused():
     heads, P, N, G, T, seqs = 2, 8, 16, 1, 5, 3
     inner = heads * P
