@@ -3,19 +3,17 @@
 // One CTA owns a tile of 128 query rows that share one kv head (row r = token r / G, head r % G of the
 // group, G = heads / kv_heads) and walks the cache in blocks of 128 keys (two pages). Per block:
 //
-//   warp 0   TMA producer: the block's K and V pages (64 x 64 elements each, 128-byte swizzle) into a
-//            ring of four stages (each group works on one and waits for the next). Pages past the sequence's end, pages a window has given back, and the
-//            rows of the last page past the sequence's length are zeroed in shared memory (V only: a
-//            masked score becomes a weight of exactly 0, and 0 times stale bits must stay 0).
-//   warp 1 and warp 10: one lane of each issues S = Q K^T and O += P V:
-//   warp 1   one thread issues S = Q K^T (tcgen05.mma, M 128, N 128, K 16 x D / 16, Q and K K-major) into
-//            one of two S buffers in tensor memory, and O += P V (M 128, N D, K 16 x 8, P K-major from
-//            shared memory, V MN-major: the pages' own layout) into the output, which stays in tensor memory.
-//   warps 2-9 softmax, two threads a query row (64 keys of the block each): tcgen05.ld of S, mask (causal,
-//            window), running maximum and sum in float32 with base-2 exponentials, P as bfloat16 into
-//            shared memory (swizzled by hand as TMA would have). When a row's maximum moves, its threads
-//            rescale their halves of its output in tensor memory (tcgen05.ld, multiply, tcgen05.st) before
-//            they hand the block's P over; the output is read once, at the end.
+//   warp 0         TMA producer: the block's K and V pages (64 x 64 elements each, 128-byte swizzle) into a ring of four
+//                  stages (each group works on one and waits for the next). Pages past the sequence's end, pages a window has
+//                  given back, and the rows of the last page past the sequence's length are zeroed in shared memory (V only: a
+//                  masked score becomes a weight of exactly 0, and 0 times stale bits must stay 0).
+//   warps 1, 10    one elected lane of warp 1 issues S = Q K^T (tcgen05.mma, M 128, N 128, K 16 x D / 16, Q and K K-major) into
+//                  the S buffer of the block's group in tensor memory, one of warp 10 O += P V (M 128, N D, K 16 x 8, P K-major
+//                  from shared memory, V MN-major: the pages' own layout) into the group's output, which stays in tensor memory.
+//   warps 2-9      softmax, in two groups of four warps on alternate blocks, a thread a query row: tcgen05.ld of S, mask (causal,
+//                  window), running maximum and sum in float32 with base-2 exponentials, P as bfloat16 into shared memory
+//                  (swizzled by hand as TMA would have). When a row's maximum moves, its thread rescales its row of the group's
+//                  output in tensor memory (tcgen05.ld, multiply, tcgen05.st); the groups' outputs are merged at the end.
 //
 // A group's next S is issued as soon as it has read its scores, and runs under its softmax. A group's weights wait for its previous
 // P V: it reads the memory they are written to. Measured on B200 (us; 16 heads over 8): 8,192 tokens 314 -> 273, behind 8,192 more 782
