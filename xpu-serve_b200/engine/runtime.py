@@ -95,8 +95,8 @@ class Runtime:
         # Products with more rows. "auto": this library's tcgen05 kernel where it fuses an epilogue that the
         # library product cannot (the gate/up product with its activation, from 512 tokens on), cuBLAS elsewhere.
         # Measured on B200, L2 flushed, us, this kernel against the library's. Gate/up (against product and activation
-        # kernel): N 16384 K 2048 at 512, 2,048 and 8,192 tokens 43, 104 and 371 against 40, 118 and 415; N 13312 K 1024
-        # 33, 70 and 221 against 25, 67 and 222. (Where it is level or behind, below 2,048 tokens, the fused form
+        # kernel): N 16384 K 2048 at 512, 1,024, 2,048 and 8,192 tokens 41, 66, 105 and 380 against 40, 68, 120 and 417; N 13312
+        # K 1024 27, 35, 57 and 180 against 25, 38, 67 and 222. (Where it is level or behind, below 1,024 tokens, the fused form
         # still rounds once less: gate and up stay float32 until the activation.) in_proj, q/k/v, out_proj and down: the
         # library is faster at every size, 512 tokens by 1.3 to 2.6 times, 2,048 by 1.1 to 1.6, 8,192 by 1.04 to 1.2,
         # mostly because it cuts the last, partly filled wave of tiles finer. "tcgen05": every such product on this

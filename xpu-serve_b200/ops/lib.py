@@ -1117,11 +1117,11 @@ def moe_few_tokens(experts: int, up_rows: int, down_rows: int) -> int:
     """Up to how many tokens experts with so many rows in their two weights take `moe_few_rows` instead of plan, gather and the
     padded tcgen05 products. 16 in general; MOE_FEW_TOKENS where the two products have at most 1,024 CTAs of 32 weight rows.
     Measured on B200, routed units from ids to the combined rows, us, this way against the other: 16 of 1,024 at width 2,048, top 4: 8
-    tokens 58 against 76, 16 tokens 62 against 80, 17 tokens 101 against 78 (from 17 on a product carries four groups of eight columns, in
-    156 registers, one CTA an SM). 64 of 512, top 8: 83 against 109, 109 against 123, 198 against 121. 17 to 32 tokens with few CTAs:
-    8 of 256 at width 512 15 against 41, 16 of 512 at width 1,024 (1,024 CTAs) 42 against 51, 8 of 1,024 at width 2,048 (1,024) 60 against 65;
-    with 1,280 and more it depends: 64 against 76, 95 against 88, 67 against 64. The one size where it lost at 9 to 16 tokens: 16 of 2,816 at
-    width 4,096 (1.1 GB of weights), 239 against 229."""
+    tokens 49 against 63, 16 tokens 58 against 68, 17 tokens 99 against 65 (from 17 on a product carries four groups of eight columns, in
+    156 registers, one CTA an SM). 64 of 512, top 8: 75 against 104, 89 against 115, 194 against 113. 17 to 32 tokens with few CTAs:
+    8 of 256 at width 512 15 against 28; at the line itself the two are close, 16 of 512 at width 1,024 (1,024 CTAs) 42 against 39, 8 of
+    1,024 at width 2,048 (1,024) 60 against 53. The one size where it lost at 9 to 16 tokens: 16 of 2,816 at width 4,096 (1.1 GB of
+    weights), 241 against 227."""
     return MOE_FEW_TOKENS if experts * (up_rows + down_rows) <= 32 * 1024 else 16
 
 
